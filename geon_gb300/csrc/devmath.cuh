@@ -40,6 +40,7 @@
 //   software is freely granted, provided that this notice
 //   is preserved.
 #pragma once
+#include "softfp.cuh"
 
 namespace geon {
 namespace dm {
@@ -74,14 +75,41 @@ constexpr double EX_Q3 = -0x1.4ce199eaadbb7p-14;
 constexpr double EX_Q4 = 0x1.0cfca86e65239p-18;
 constexpr double EX_Q5 = -0x1.afdb76e09c32dp-23;
 
+// k = rint(x * TWO_OVER_PI) and q = k mod 4 (exactly: the CPU oracle computes
+// k - 4 floor(k / 4)) of a finite x. Polar angles are in [0, pi], where k is 0,
+// 1 or 2 and the high word of x tells which: the product crosses 1/2 and 3/2
+// at pi/4 = 0x3fe921fb54442d18 and 3 pi/4 = 0x4002d97c7f3321d2 to a few ulp, so
+// only the two high words that hold a crossing need the product itself. That
+// keeps a multiplication, a rounding and a conversion (51 cycles of the FP64
+// pipe per warp) out of the common case.
+__device__ __forceinline__ void quadrant(double x, double& k, int& q) {
+  const unsigned hx = sf::hi_of(x);
+  if (hx < 0x400f6a7au && hx != 0x3fe921fbu && hx != 0x4002d97cu) {  // 0 <= x < 5 pi/4
+    q = (hx > 0x3fe921fbu ? 1 : 0) + (hx > 0x4002d97cu ? 1 : 0);
+    k = sf::from_words(q == 0 ? 0u : (q == 1 ? 0x3ff00000u : 0x40000000u), 0u);
+    return;
+  }
+  k = rint(x * TWO_OVER_PI);
+  // Below 2^52 the integer conversion is exact and two's-complement & 3 is the
+  // mathematical residue; above it k is an even integer and the double formula
+  // is exact, and no integer type would hold k.
+  if (fabs(k) < 0x1p52) {
+    q = (int)(__double2ll_rn(k) & 3);
+  } else {
+    q = (int)(k - 4.0 * floor(k * 0.25));
+  }
+}
+
 __device__ __forceinline__ void sincos_det(double x, double* sp, double* cp) {
-  if (!isfinite(x)) {
+  if (!sf::finite(x)) {
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
     *sp = nan;
     *cp = nan;
     return;
   }
-  const double k = rint(x * TWO_OVER_PI);
+  double k;
+  int q;
+  quadrant(x, k, q);
   const double r1 = fma(-k, PIO2_1, x);
   const double t = fma(-k, PIO2_2, r1);
   const double d = r1 - t;
@@ -96,7 +124,8 @@ __device__ __forceinline__ void sincos_det(double x, double* sp, double* cp) {
   ps = fma(ps, z, S5);
   ps = fma(ps, z, S3);
   const double tz = t * z;
-  const double sv = t + fma(tz, ps, tl * fma(-0.5, z, 1.0));
+  const double wc = fma(-0.5, z, 1.0);  // 1 - z / 2 (the product is exact)
+  const double sv = t + fma(tz, ps, tl * wc);
   double pc = C18;
   pc = fma(pc, z, C16);
   pc = fma(pc, z, C14);
@@ -105,20 +134,8 @@ __device__ __forceinline__ void sincos_det(double x, double* sp, double* cp) {
   pc = fma(pc, z, C8);
   pc = fma(pc, z, C6);
   pc = fma(pc, z, C4);
-  const double hz = 0.5 * z;
-  const double wc = 1.0 - hz;
   const double zl = fma(t, t, -z);
-  const double cv = wc + (((1.0 - wc) - hz) + (fma(z * z, pc, -0.5 * zl) - tl * t));
-  // q = k mod 4 in [0, 4), exactly (the CPU oracle computes k - 4 floor(k / 4)).
-  // Below 2^52 the integer conversion is exact and two's-complement & 3 is the
-  // mathematical residue; above it k is an even integer and the double formula
-  // is exact, and no integer type would hold k.
-  int q;
-  if (fabs(k) < 0x1p52) {
-    q = (int)(__double2ll_rn(k) & 3);
-  } else {
-    q = (int)(k - 4.0 * floor(k * 0.25));
-  }
+  const double cv = wc + (fma(-0.5, z, 1.0 - wc) + (fma(z * z, pc, -0.5 * zl) - tl * t));
   double s, c;
   if (q == 0) { s = sv; c = cv; }
   else if (q == 1) { s = cv; c = -sv; }
@@ -171,7 +188,7 @@ __device__ __forceinline__ double expm1_det(double x) {
   const double z2 = z * z, z4 = z2 * z2;
   const double R = fma(z4, fma(z, EX_Q5, EX_Q4), fma(z2, fma(z, EX_Q3, EX_Q2), fma(z, EX_Q1, 1.0)));
   const double t = fma(-R, hfx, 3.0);
-  double e = z * ((R - t) / fma(-x, t, 6.0));
+  double e = z * sf::div(R - t, fma(-x, t, 6.0));
   if (k == 0) return x - fma(x, e, -z);
   e = fma(x, e - c, -c) - z;
   if (k == -1) return fma(0.5, x - e, -0.5);
@@ -189,15 +206,17 @@ __device__ __forceinline__ double tanh_det(double x) {
   const unsigned jx = hi_word(x), ix = jx & 0x7fffffffu;
   const bool neg = (jx >> 31) != 0;
   if (ix >= 0x7ff00000u) return neg ? 1.0 / x - 1.0 : 1.0 / x + 1.0;  // NaN, +-inf
-  double z = 1.0;                           // |x| >= 22
-  if (ix < 0x40360000u) {
+  // The published method answers 1 from |x| = 22 on; from 19.0625 on its formula
+  // gives 1 already (2 / (expm1(38.125) + 2) = 5.541e-17 is below 2^-54).
+  double z = 1.0;
+  if (ix < 0x40331000u) {
     if (ix < 0x3c800000u) return x * (1.0 + x);  // |x| < 2^-55
     if (ix >= 0x3ff00000u) {
       const double m = expm1_det(2.0 * fabs(x));
-      z = 1.0 - 2.0 / (m + 2.0);
+      z = 1.0 - sf::div(2.0, m + 2.0);
     } else {
       const double m = expm1_det(-2.0 * fabs(x));
-      z = -m / (m + 2.0);
+      z = -sf::div(m, m + 2.0);
     }
   }
   return neg ? -z : z;

@@ -90,7 +90,7 @@ class Gen:
     def div(self, a, b):
         if a.is_zero():
             return ZERO
-        return self.tmp(f"{a.c()} / {b.c()}")
+        return self.tmp(f"sf::rcp({b.c()})" if a.const == 1.0 else f"sf::div({a.c()}, {b.c()})")
 
     def acc(self, s, t):
         """s += t for a sum that started at 0.0."""
@@ -321,7 +321,7 @@ def op_counts():
             if not m:
                 continue
             expr = m.group(1)
-            for sym, key in ((" * ", "mul"), (" + ", "add"), (" - ", "sub"), (" / ", "div")):
+            for sym, key in ((" * ", "mul"), (" + ", "add"), (" - ", "sub"), ("sf::div(", "div"), ("sf::rcp(", "div")):
                 if sym in expr:
                     ops[key] += 1
                     break

@@ -92,10 +92,10 @@ __device__ __forceinline__ bool inv4(const double a[16], double out[16]) {
 __device__ __forceinline__ void alc_g00_g01(const MetricDesc& M, const double x[4], double* g00, double* g01) {
   const double R = M.p[0], s = M.p[1], v = M.p[2], ship_x = M.p[3];
   const double dx = x[1] - ship_x, dy = x[2], dz = x[3];
-  const double r_s = sqrt(dx * dx + dy * dy + dz * dz);
-  const double t_plus = dm::tanh_det((r_s + R) / s);
-  const double t_minus = dm::tanh_det((r_s - R) / s);
-  const double f = (t_plus - t_minus) / M.alc_denom;
+  const double r_s = sf::root(dx * dx + dy * dy + dz * dz);
+  const double t_plus = dm::tanh_det(sf::div(r_s + R, s));
+  const double t_minus = dm::tanh_det(sf::div(r_s - R, s));
+  const double f = sf::div(t_plus - t_minus, M.alc_denom);
   *g00 = -1.0 + v * v * f * f;
   *g01 = -v * f;
 }
@@ -413,17 +413,17 @@ __device__ __forceinline__ int metric_terminate(const MetricDesc& M, const doubl
     return r2 > 1e6 ? TERM_ESCAPED : TERM_NONE;
   } else if (K == KIND_SCHWARZSCHILD) {
     const double r = x[1];
-    if (!isfinite(r)) return TERM_DIVERGED;
+    if (!sf::finite(r)) return TERM_DIVERGED;
     if (r < M.capture_r) return TERM_CAPTURED;
     if (r > M.escape_r) return TERM_ESCAPED;
     return TERM_NONE;
   } else if (K == KIND_ALCUBIERRE) {
     const double r2 = x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
-    if (!isfinite(r2)) return TERM_DIVERGED;
+    if (!sf::finite(r2)) return TERM_DIVERGED;
     return r2 > 1e6 ? TERM_ESCAPED : TERM_NONE;
   } else if (K == KIND_MORRIS_THORNE) {
     const double l = x[1];
-    if (!isfinite(l)) return TERM_DIVERGED;
+    if (!sf::finite(l)) return TERM_DIVERGED;
     return fabs(l) > 1000.0 ? TERM_ESCAPED : TERM_NONE;
   } else {  // sampled metric: leaving the grid ends the ray (below the inner radius of a spherical chart: Captured)
     if (!isfinite(x[1]) || !isfinite(x[2]) || !isfinite(x[3])) return TERM_DIVERGED;
@@ -485,34 +485,32 @@ __device__ __forceinline__ bool geodesic_rhs(const MetricDesc& M, const double y
     // schwarzschild.rs:61-107 fused with the sum; only the nonzero entries
     // contribute (alpha-major, beta-minor order kept).
     const double r = y[1], theta = y[2], m = M.p[0];
-    const double f = 1.0 - 2.0 * m / r;
+    const double f = 1.0 - sf::div(2.0 * m, r);
     double sin_t, cos_t;
     dm::sincos_det(theta, &sin_t, &cos_t);
     const double rr = r * r;
-    const double rrf = rr * f;
-    const double gtr = m / rrf;            // Gamma^t_tr = Gamma^t_rt
-    const double g_r_tt = m * f / rr;      // Gamma^r_tt
-    const double g_r_rr = -gtr;            // -m/(r r f) == -(m/(r r f))
-    const double r2m = r - 2.0 * m;
-    const double g_r_thth = -r2m;          // Gamma^r_thth
-    const double g_r_phph = -r2m * sin_t * sin_t;
-    const double ir = 1.0 / r;             // Gamma^th_rth, Gamma^ph_rph
-    const double g_th_phph = -sin_t * cos_t;
-    const double cot = fabs(sin_t) < 1e-8 ? 0.0 : cos_t / sin_t;
+    const double gtr = sf::div(m, rr * f);      // Gamma^t_tr = Gamma^t_rt = -Gamma^r_rr
+    const double g_r_tt = sf::div(m * f, rr);   // Gamma^r_tt
+    const double r2m = r - 2.0 * m;             // -Gamma^r_thth
+    const double ir = sf::rcp(r);               // Gamma^th_rth, Gamma^ph_rph
+    const double cot = sf::below(sin_t, 1e-8) ? 0.0 : sf::div(cos_t, sin_t);
+    // Products shared between the sums; a negated entry is a subtracted term
+    // (x + (-y) is x - y, and (-a) b c is -((a b) c), bit for bit).
+    const double gp1 = gtr * p1, irp1 = ir * p1;
     double s;
     s = plus_zero(gtr * p0 * p1);
-    s += gtr * p1 * p0;
+    s += gp1 * p0;
     k[4] = -s;
     s = plus_zero(g_r_tt * p0 * p0);
-    s += g_r_rr * p1 * p1;
-    s += g_r_thth * p2 * p2;
-    s += g_r_phph * p3 * p3;
+    s -= gp1 * p1;
+    s -= r2m * p2 * p2;
+    s -= r2m * sin_t * sin_t * p3 * p3;
     k[5] = -s;
-    s = plus_zero(ir * p1 * p2);
+    s = plus_zero(irp1 * p2);
     s += ir * p2 * p1;
-    s += g_th_phph * p3 * p3;
+    s -= sin_t * cos_t * p3 * p3;
     k[6] = -s;
-    s = plus_zero(ir * p1 * p3);
+    s = plus_zero(irp1 * p3);
     s += cot * p2 * p3;
     s += ir * p3 * p1;
     s += cot * p3 * p2;
@@ -540,32 +538,47 @@ __device__ __forceinline__ bool geodesic_rhs(const MetricDesc& M, const double y
 }
 
 // Classical RK4 (integrator.rs:16-40) with the reference's grouping:
-// y + (0.5*h)*k, y + h*k3, and y + (h/6)*(((k1 + 2 k2) + 2 k3) + k4).
+// y + (0.5*h)*k, y + h*k3, and y + (h/6)*(((k1 + 2 k2) + 2 k3) + k4). The
+// stages run in a loop: the right-hand side is a thousand instructions and more,
+// and one copy of it stays in the instruction cache. k1 + 2 k2 is one fused
+// operation with the same bits, since 2 k2 is exact; only where 2 k2 or 2 k3
+// overflows (or is not a number) could the two differ, and there the
+// reference's sum is infinite or NaN, so *finite reports it with the
+// non-finite results (geodesic.rs:89-100).
 template <int K>
 __device__ __forceinline__ bool rk4_step(const MetricDesc& M, const double y[8], double h,
-                                         double half_h, double sixth, double out[8]) {
+                                         double half_h, double sixth, double out[8], bool* finite) {
   double k[8], acc[8], ys[8];
-  bool ok = geodesic_rhs<K>(M, y, k);
+  unsigned big = 0;  // the largest |high word| of k2 and k3, times 2
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    acc[i] = k[i];
-    ys[i] = y[i] + half_h * k[i];
+  for (int i = 0; i < 8; ++i) ys[i] = y[i];
+  bool ok = true;
+#pragma unroll 1
+  for (int stage = 0; stage < 3; ++stage) {
+    ok &= geodesic_rhs<K>(M, ys, k);
+    const double c = stage < 2 ? half_h : h;
+    if (stage == 0) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = k[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        acc[i] = fma(2.0, k[i], acc[i]);
+        const unsigned a = 2u * sf::hi_of(k[i]);
+        big = a > big ? a : big;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ys[i] = y[i] + c * k[i];
   }
   ok &= geodesic_rhs<K>(M, ys, k);
+  bool fin = big < 2u * 0x7fe00000u;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    acc[i] = acc[i] + 2.0 * k[i];
-    ys[i] = y[i] + half_h * k[i];
+    out[i] = y[i] + sixth * (acc[i] + k[i]);
+    fin &= sf::finite(out[i]);
   }
-  ok &= geodesic_rhs<K>(M, ys, k);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    acc[i] = acc[i] + 2.0 * k[i];
-    ys[i] = y[i] + h * k[i];
-  }
-  ok &= geodesic_rhs<K>(M, ys, k);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) out[i] = y[i] + sixth * (acc[i] + k[i]);
+  *finite = fin;
   return ok;
 }
 

@@ -1,0 +1,235 @@
+// Correctly rounded FP64 division, reciprocal and square root in 32-bit integer
+// arithmetic.
+//
+// GB300 executes FP64 at 1/64 of its integer and FP32 rate: a warp holds the
+// FP64 pipe of an SM for 16-19 cycles per DADD, DMUL, DFMA or DSETP, and an
+// IEEE division for 141 (square root 143, reciprocal 86; a division whose
+// numerator is zero takes the slow path: 350), measured with independent
+// chains at 16 warps per SM. The integer pipes of the same kernels are idle.
+// The functions here return the same bits as the IEEE operations in 29 (div),
+// 32 (root) and 27 (rcp) cycles that leave the FP64 pipe free, by digit
+// recurrence on the 53-bit significands:
+//   * a digit is the remainder's leading word times a hardware FP32 reciprocal
+//     (or reciprocal square root) of the divisor, ~22 bits at a time; the
+//     remainder after each digit is formed exactly (modulo 2^64, which holds it);
+//   * after three digits the quotient (root) is known to within one unit and
+//     its remainder is exact, so comparing twice the remainder with the divisor
+//     (the remainder with the root) rounds to nearest. Neither a quotient nor a
+//     root of FP64 numbers can be a tie.
+// Digit recurrence with a reciprocal estimate: M. Ercegovac, T. Lang, "Division
+// and Square Root: Digit-Recurrence Algorithms and Implementations" (1994),
+// very-high-radix division by prescaling; the error bounds are beside the code.
+// Operands outside [2^-255, 2^257) (zero, subnormal, huge, infinite, NaN) go to
+// the hardware operation; a zero numerator is answered directly.
+//
+// Host and device code: the CPU tests compile it with g++ and compare it with
+// the host's division and square root, moving the estimates by their error.
+#pragma once
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+
+#ifdef __CUDACC__
+#define GEON_SF __device__ __forceinline__
+#else
+#define GEON_SF inline
+#endif
+
+namespace geon {
+namespace sf {
+
+GEON_SF uint64_t bits(double x) {
+#ifdef __CUDA_ARCH__
+  return (uint64_t)__double_as_longlong(x);
+#else
+  uint64_t u;
+  memcpy(&u, &x, 8);
+  return u;
+#endif
+}
+GEON_SF double from_words(uint32_t hi, uint32_t lo) {
+#ifdef __CUDA_ARCH__
+  return __hiloint2double((int)hi, (int)lo);
+#else
+  const uint64_t u = ((uint64_t)hi << 32) | lo;
+  double x;
+  memcpy(&x, &u, 8);
+  return x;
+#endif
+}
+GEON_SF uint32_t hi_of(double x) {
+#ifdef __CUDA_ARCH__
+  return (uint32_t)__double2hiint(x);
+#else
+  return (uint32_t)(bits(x) >> 32);
+#endif
+}
+GEON_SF uint32_t lo_of(double x) {
+#ifdef __CUDA_ARCH__
+  return (uint32_t)__double2loint(x);
+#else
+  return (uint32_t)bits(x);
+#endif
+}
+
+// x is neither infinite nor NaN, without a DSETP
+GEON_SF bool finite(double x) { return (hi_of(x) & 0x7ff00000u) != 0x7ff00000u; }
+
+// |x| < t for a positive t (false for NaN): magnitudes order like their bits
+GEON_SF bool below(double x, double t) { return (bits(x) & 0x7fffffffffffffffull) < bits(t); }
+
+// Estimates of 1/x (x in [1, 2]) and 1/sqrt(x) (x in [1, 4]) as FP32 bits,
+// relative error at most 2^-23 and 2^-22.4 (PTX rcp.approx, rsqrt.approx). On
+// the host `est_error` moves them by units in the last place (tests).
+#ifdef __CUDA_ARCH__
+GEON_SF uint32_t rcp_bits(uint32_t x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(x)));
+  return __float_as_uint(r);
+}
+GEON_SF uint32_t rsqrt_bits(uint32_t x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(x)));
+  return __float_as_uint(r);
+}
+GEON_SF uint32_t umulhi(uint32_t a, uint32_t b) { return __umulhi(a, b); }
+GEON_SF int32_t smulhi(int32_t a, int32_t b) { return __mulhi(a, b); }
+#else
+inline int& est_error() {
+  static int e = 0;
+  return e;
+}
+inline uint32_t rcp_bits(uint32_t x) {
+  float f, r;
+  memcpy(&f, &x, 4);
+  r = (float)(1.0 / (double)f);
+  uint32_t u;
+  memcpy(&u, &r, 4);
+  return u + est_error();
+}
+inline uint32_t rsqrt_bits(uint32_t x) {
+  float f, r;
+  memcpy(&f, &x, 4);
+  r = (float)(1.0 / sqrt((double)f));
+  uint32_t u;
+  memcpy(&u, &r, 4);
+  return u + est_error();
+}
+inline uint32_t umulhi(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
+inline int32_t smulhi(int32_t a, int32_t b) { return (int32_t)(((int64_t)a * b) >> 32); }
+#endif
+
+// Zero exactly when |x| (its high word) is in [2^-255, 2^257), else not zero.
+GEON_SF uint32_t outside(uint32_t hi) { return (hi * 2u + 0xA0000000u) & 0xC0000000u; }
+
+GEON_SF uint64_t pack(uint32_t hi, uint32_t lo) { return ((uint64_t)hi << 32) | lo; }
+
+// n - d * b modulo 2^64, d signed
+GEON_SF uint64_t minus_product(uint64_t n, int32_t d, uint64_t b) {
+  const uint32_t nd = (uint32_t)-d;
+  uint64_t r = n + (uint64_t)nd * (uint32_t)b;
+  uint32_t h = (uint32_t)(r >> 32) + nd * (uint32_t)(b >> 32);
+  if (nd >> 31) h -= (uint32_t)b;  // nd as a signed factor
+  return pack(h, (uint32_t)r);
+}
+
+// An FP32 estimate in [0.5, 1) as 2^31 times its value (ends clamped).
+GEON_SF uint32_t fixed31(uint32_t r) {
+  r = r > 0x3f000000u ? r : 0x3f000000u;
+  r = r < 0x3f7fffffu ? r : 0x3f7fffffu;
+  return ((r << 7) & 0x3fffffffu) | 0x40000000u;
+}
+
+// Significand (53 bits) of a / b rounded to nearest, for significands A' in
+// [B, 2B) and B in [2^52, 2^53). Y = 2^31 times an estimate of 2^52 / B with
+// relative error e at most 2^-21.7 (two units in the last place of the
+// estimate, 2^-22, and its argument's 2^-24; the hardware's is one unit).
+//   d1 ~ (A'/B) 2^30 < 2^31: error < 2^9.3 + 2  =>  |R1| < 2^9.4 B < 2^62.4
+//   d2 ~ R1/B 2^19, |d2| < 2^28.4: error < 2^6.7 + 2  =>  |R2| < 2^6.8 B
+//   d3 ~ floor(R2/B 2^3): error in [0, 1] and a part in 2^11 either way, so the
+// quotient is Q = d1 2^22 + d2 2^3 + d3 plus R3 / B with R3 in (-B/2^11, 1.01 B).
+GEON_SF uint64_t quotient(uint64_t A, uint64_t B, uint32_t Y) {
+  const uint32_t d1 = umulhi((uint32_t)(A >> 22), Y << 1);
+  uint64_t R = (A << 30) - ((uint64_t)d1 * (uint32_t)B + ((uint64_t)(d1 * (uint32_t)(B >> 32)) << 32));
+  const int32_t d2 = smulhi((int32_t)(R >> 32), (int32_t)Y);
+  R = minus_product(R << 19, d2, B);
+  const int32_t d3 = smulhi((int32_t)(R >> 32), (int32_t)Y) >> 16;
+  R = minus_product(R << 3, d3, B);
+  uint64_t Q = ((uint64_t)d1 << 22) + (uint64_t)((int64_t)d2 * 8 + d3);
+  if ((int64_t)(2 * R - B) > 0) ++Q;  // 2 R3 > B
+  return Q;
+}
+
+// 2^31 times the estimate of 2^52 / B (the argument rounded to 24 bits).
+GEON_SF uint32_t reciprocal_estimate(uint64_t B) {
+  const uint32_t f = 0x3f800000u + ((uint32_t)((B + (1u << 28)) >> 29) - (1u << 23));
+  return fixed31(rcp_bits(f));
+}
+
+// a / b, rounded to nearest: the bits of the IEEE division.
+GEON_SF double div(double a, double b) {
+  const uint32_t ah = hi_of(a), al = lo_of(a), bh = hi_of(b), bl = lo_of(b);
+  if (outside(bh) | outside(ah)) {
+    if ((((ah << 1) | al) | outside(bh)) == 0u) return from_words((ah ^ bh) & 0x80000000u, 0u);  // +-0 / b
+    return a / b;
+  }
+  const uint32_t am = (ah & 0xfffffu) | 0x100000u, bm = (bh & 0xfffffu) | 0x100000u;
+  const uint64_t B = pack(bm, bl);
+  uint64_t A = pack(am, al);
+  const uint32_t less = A < B ? 1u : 0u;
+  A <<= less;
+  const uint64_t Q = quotient(A, B, reciprocal_estimate(B));
+  // exponents and signs: (ah - am) and (bh - bm) hold sign, exponent - 1
+  const uint32_t h = (uint32_t)(Q >> 32) + (ah - am) - (bh - bm) + (1022u << 20) - (less << 20);
+  return from_words(h, (uint32_t)Q);
+}
+
+// 1 / b
+GEON_SF double rcp(double b) {
+  const uint32_t bh = hi_of(b), bl = lo_of(b);
+  if (outside(bh)) return 1.0 / b;
+  const uint32_t bm = (bh & 0xfffffu) | 0x100000u;
+  const uint64_t B = pack(bm, bl);
+  const uint32_t less = (bl | (bm ^ 0x100000u)) ? 1u : 0u;  // B is not a power of two
+  const uint64_t Q = quotient((uint64_t)1 << (52 + less), B, reciprocal_estimate(B));
+  const uint32_t h = (uint32_t)(Q >> 32) + (1022u << 20) - (bh - bm) + (1022u << 20) - (less << 20);
+  return from_words(h, (uint32_t)Q);
+}
+
+// sqrt(a), rounded to nearest: the bits of the IEEE square root. With n in
+// [1, 4) the significand (times 2 for an odd exponent), A = n 2^52, and y the
+// estimate of 1/sqrt(n) (relative error at most 2^-22.9, argument 2^-24, clamp
+// 2^-24: together 2^-22), Y = 2^31 y:
+//   S1 ~ sqrt(n) 2^30: error < 2^9.1, R1 = n 2^60 - S1^2, |R1| < 2^41.1
+//   d2 ~ R1 y 2^-12 (half the remainder over the root, 2^19 times finer):
+//     T = S1 2^19 + d2 ~ sqrt(n) 2^49: error < 2^7.3, R2 = n 2^98 - T^2, |R2| < 2^58.3
+//   d3 = floor(R2 y 2^-47): S = 2^3 T + d3, so sqrt(n) 2^52 lies in
+//     [S, S + 1] and a part in 2^10 either way; it rounds up when its remainder
+//     N - S^2 (N = n 2^104) exceeds S.
+GEON_SF double root(double a) {
+  const uint32_t ah = hi_of(a), al = lo_of(a);
+  if (outside(ah) | (ah >> 31)) {
+    return sqrt(a);
+  }
+  const uint32_t am = (ah & 0xfffffu) | 0x100000u;
+  const uint32_t odd = ((ah >> 20) & 1u) ^ 1u;  // the unbiased exponent is odd
+  const uint64_t A = pack(am, al) << odd;
+  // n to 24 bits as FP32
+  const uint32_t fb = 0x3f000000u + (odd << 23) + (uint32_t)(pack(am, al) >> 29);
+  const uint32_t Y = fixed31(rsqrt_bits(fb));
+  const uint32_t S1 = umulhi((uint32_t)(A >> 22), Y << 1);
+  const uint64_t R1 = (A << 8) - (uint64_t)S1 * S1;
+  const int32_t d2 = smulhi((int32_t)((int64_t)R1 >> 11), (int32_t)Y);
+  const uint64_t T = ((uint64_t)S1 << 19) + (uint64_t)(int64_t)d2;
+  const uint64_t R2 = minus_product(R1 << 38, d2, (T << 1) - (uint64_t)(int64_t)d2);
+  const int32_t d3 = smulhi((int32_t)((int64_t)R2 >> 28), (int32_t)Y) >> 18;
+  const uint64_t S = (T << 3) + (uint64_t)(int64_t)d3;
+  // N - S^2 = R2 2^6 - d3 (2^4 T + d3)
+  const uint64_t R3 = minus_product(R2 << 6, d3, (T << 4) + (uint64_t)(int64_t)d3);
+  const uint64_t M = S + ((int64_t)(R3 - S) > 0 ? 1u : 0u);
+  const uint32_t h = (uint32_t)(M >> 32) + ((((ah >> 20) - odd + 1021u) >> 1) << 20);
+  return from_words(h, (uint32_t)M);
+}
+
+}  // namespace sf
+}  // namespace geon

@@ -125,6 +125,20 @@ __device__ __forceinline__ void store_ray(const TraceLaunch& L, int64_t ray, int
 }
 
 constexpr int TRACE_BLOCK = 128;
+// Block size of the FP64 trace kernels: one warp. A warp is the unit of work
+// (nothing in the loop is shared by a block), and the FP64 units, one per SM
+// quarter, set the time, so the warps have to spread over all SMs: 65536 rays
+// in blocks of four warps put 3 or 4 blocks on an SM (16 warps against 13.5 on
+// average), 5184 rays use 41 of the 152 SMs.
+constexpr int FP64_BLOCK = 32;
+// Blocks of a persistent FP64 grid over n rays (the caller's reserve counts
+// slots of TRACE_BLOCK threads).
+inline int fp64_grid(int sms, int per_sm, float reserve, int64_t n) {
+  const int64_t slots = persistent_slots(sms, per_sm, reserve * (float)TRACE_BLOCK / (float)FP64_BLOCK);
+  const int64_t need = (n + FP64_BLOCK - 1) / FP64_BLOCK;
+  const int64_t grid = need < slots ? need : slots;
+  return (int)(grid < 1 ? 1 : grid);
+}
 // Steps a lane takes between two refills of its warp: the ballots and the
 // queue test are paid once per TRACE_INNER steps; a lane whose ray ends inside
 // the group waits at most TRACE_INNER - 1 steps for the next ray.

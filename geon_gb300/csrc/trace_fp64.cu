@@ -30,10 +30,8 @@ struct Fp64Stepper {
   __device__ __forceinline__ int terminate(const TraceLaunch& L) const { return metric_terminate<K>(L.M, y); }
   __device__ __forceinline__ int step(const TraceLaunch& L) {
     double yn[8];
-    singular |= !rk4_step<K>(L.M, y, L.step, L.half_step, L.sixth, yn);
-    bool finite = true;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) finite &= isfinite(yn[i]);
+    bool finite;
+    singular |= !rk4_step<K>(L.M, y, L.step, L.half_step, L.sixth, yn, &finite);
     if (!finite) return STEP_NONFINITE;
 #pragma unroll
     for (int i = 0; i < 8; ++i) y[i] = yn[i];
@@ -89,17 +87,14 @@ struct Fp64StepperAny {
   }
   __device__ __forceinline__ int step(const TraceLaunch& L) {
     double yn[8];
-    bool ok;
+    bool ok, finite;
     switch (kind) {
-      case KIND_SCHWARZSCHILD: ok = rk4_step<KIND_SCHWARZSCHILD>(L.M, y, L.step, L.half_step, L.sixth, yn); break;
-      case KIND_ALCUBIERRE: ok = rk4_step<KIND_ALCUBIERRE>(L.M, y, L.step, L.half_step, L.sixth, yn); break;
-      case KIND_MORRIS_THORNE: ok = rk4_step<KIND_MORRIS_THORNE>(L.M, y, L.step, L.half_step, L.sixth, yn); break;
-      default: ok = rk4_step<KIND_MINKOWSKI>(L.M, y, L.step, L.half_step, L.sixth, yn); break;
+      case KIND_SCHWARZSCHILD: ok = rk4_step<KIND_SCHWARZSCHILD>(L.M, y, L.step, L.half_step, L.sixth, yn, &finite); break;
+      case KIND_ALCUBIERRE: ok = rk4_step<KIND_ALCUBIERRE>(L.M, y, L.step, L.half_step, L.sixth, yn, &finite); break;
+      case KIND_MORRIS_THORNE: ok = rk4_step<KIND_MORRIS_THORNE>(L.M, y, L.step, L.half_step, L.sixth, yn, &finite); break;
+      default: ok = rk4_step<KIND_MINKOWSKI>(L.M, y, L.step, L.half_step, L.sixth, yn, &finite); break;
     }
     singular |= !ok;
-    bool finite = true;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) finite &= isfinite(yn[i]);
     if (!finite) return STEP_NONFINITE;
 #pragma unroll
     for (int i = 0; i < 8; ++i) y[i] = yn[i];
@@ -112,7 +107,7 @@ struct Fp64StepperAny {
   }
 };
 
-__global__ void __launch_bounds__(TRACE_BLOCK) trace_multi_fp64_kernel(const TraceLaunch* jobs, const MultiDesc D) {
+__global__ void __launch_bounds__(FP64_BLOCK) trace_multi_fp64_kernel(const TraceLaunch* jobs, const MultiDesc D) {
   trace_loop_multi<Fp64StepperAny, SRC_CAMERA, SINK_RENDER>(jobs, D);
 }
 
@@ -122,20 +117,23 @@ cudaError_t launch_trace_multi_fp64(const TraceLaunch* jobs, const MultiDesc& D,
     int dev = 0, occ = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, trace_multi_fp64_kernel, TRACE_BLOCK, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, trace_multi_fp64_kernel, FP64_BLOCK, 0);
     per_sm = occ < 1 ? 1 : occ;
   }
   const int64_t n = D.start[D.njobs];
   if (n <= 0) return cudaSuccess;
-  const int64_t slots = persistent_slots(sms, per_sm, reserve);
-  const int64_t need = (n + TRACE_BLOCK - 1) / TRACE_BLOCK;
-  const int grid = (int)(need < slots ? need : slots);
-  trace_multi_fp64_kernel<<<grid < 1 ? 1 : grid, TRACE_BLOCK, 0, s>>>(jobs, D);
+  trace_multi_fp64_kernel<<<fp64_grid(sms, per_sm, reserve, n), FP64_BLOCK, 0, s>>>(jobs, D);
   return cudaGetLastError();
 }
 
+// Bound by the FP64 pipe (16-19 cycles per warp instruction and SM). What the
+// step can do elsewhere it does: divisions and square roots in integers
+// (softfp.cuh), finiteness and magnitude tests on the high words, the quadrant
+// of theta from its high word. With one-warp blocks the Schwarzschild 256^2
+// view (r 30M, h 0.05, escape 100M) went from 247 to 151 ms, a 96 x 54
+// Alcubierre view of 5000 steps from 653 to 487 ms, bit for bit.
 template <int K, int SRC, int SINK>
-__global__ void __launch_bounds__(TRACE_BLOCK) trace_fp64_kernel(const TraceLaunch L) {
+__global__ void __launch_bounds__(FP64_BLOCK) trace_fp64_kernel(const TraceLaunch L) {
   trace_loop<Fp64Stepper<K>, K, SRC, SINK>(L);
 }
 
@@ -200,16 +198,12 @@ static cudaError_t launch_kst(const TraceLaunch& L, cudaStream_t s) {
     int dev = 0, occ = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, trace_fp64_kernel<K, SRC, SINK>, TRACE_BLOCK, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, trace_fp64_kernel<K, SRC, SINK>, FP64_BLOCK, 0);
     per_sm = occ < 1 ? 1 : occ;
   }
   // persistent grid: every resident slot, minus the blocks per SM the caller
   // keeps free for a concurrent job
-  const int64_t slots = persistent_slots(sms, per_sm, L.reserve_per_sm);
-  const int64_t need = (L.n + TRACE_BLOCK - 1) / TRACE_BLOCK;
-  int grid = (int)(need < slots ? need : slots);
-  if (grid < 1) grid = 1;
-  trace_fp64_kernel<K, SRC, SINK><<<grid, TRACE_BLOCK, 0, s>>>(L);
+  trace_fp64_kernel<K, SRC, SINK><<<fp64_grid(sms, per_sm, L.reserve_per_sm, L.n), FP64_BLOCK, 0, s>>>(L);
   return cudaGetLastError();
 }
 
