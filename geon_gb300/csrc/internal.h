@@ -32,6 +32,8 @@ struct MetricDesc {
   double capture_r;  // Schwarzschild: horizon_pad * 2.0 * mass   (schwarzschild.rs:114)
   double escape_r;   // Schwarzschild: escape_radius * mass        (schwarzschild.rs:116)
   double alc_denom;  // Alcubierre: 2.0 * tanh(R / s)               (alcubierre.rs:42)
+  double alc_flat;   // Alcubierre: beyond this r_s every metric value is flat, in FP64 and FP32
+                     // (metric_init_kernel; infinite where that is not known)
   FieldDesc f;       // GEON_FIELD only
 };
 

@@ -150,8 +150,13 @@ __device__ __forceinline__ void serve_loop(const ServeJob* __restrict__ jobs, Se
     if (__ballot_sync(FULL, slot >= 0) == 0) break;
     if (slot >= 0) {
       const TraceLaunch& L = jobs[slot].L;
+      int inner = 0;
+      if (n + TRACE_INNER <= L.max_steps && st.flat_group(L)) {  // a whole group through flat space
+        n += TRACE_INNER;
+        inner = TRACE_INNER;
+      }
 #pragma unroll 1
-      for (int inner = 0; inner < TRACE_INNER; ++inner) {
+      for (; inner < TRACE_INNER; ++inner) {
         int t = TERM_NONE;
         long long taken = n;
         if (n >= L.max_steps) {

@@ -158,6 +158,8 @@ __device__ __forceinline__ int64_t group_steps(Stepper& st, const TraceLaunch& L
   const int left = left64 < (int64_t)TRACE_INNER ? (int)left64 : TRACE_INNER;
   int done = 0, extra = 0;
   t = TERM_NONE;
+  // a whole group through flat space at once (the same steps: see the steppers)
+  if (left == TRACE_INNER && st.flat_group(L)) done = TRACE_INNER;
 #pragma unroll 1
   for (; done < left; ++done) {
     t = st.terminate(L);
