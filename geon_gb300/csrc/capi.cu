@@ -36,8 +36,9 @@ std::atomic<float> g_reserve{0.0f};
 std::atomic<double> g_rtol{1e-10};  // GEON_ADAPTIVE error tolerances
 std::atomic<double> g_atol{1e-12};
 // Mixed-kernel variant per metric kind and ray source (camera/array, equatorial),
-// chosen by geon_autotune_mixed (default 0).
-std::atomic<int> g_variant[4][2] = {{{0}, {0}}, {{0}, {0}}, {{0}, {0}}, {{0}, {0}}};
+// chosen by geon_autotune_mixed (default 0, except the equatorial source: 2, at
+// most 51 registers; the 2^20-ray sweep takes 267 ms with it, 271 without a cap).
+std::atomic<int> g_variant[4][2] = {{{0}, {0}}, {{0}, {2}}, {{0}, {0}}, {{0}, {0}}};
 // Kernels launched by this library since load (ours only; memsets excluded).
 std::atomic<unsigned long long> g_launches{0};
 inline void counted(unsigned long long n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
@@ -134,6 +135,37 @@ int make_camera(geon_metric_t m, const geon_camera* cam, int64_t spa, CameraDesc
   return GEON_OK;
 }
 
+// The mixed path's FP32 constants: each the FP64 value rounded once.
+MixedConsts mixed_consts(const MetricDesc& M, double step, double half_step, double sixth, int64_t max_steps) {
+  MixedConsts c;
+  c.m = (float)M.p[0];
+  c.two_m = (float)(2.0 * M.p[0]);
+  c.b0sq = (float)(M.p[0] * M.p[0]);
+  c.R = (float)M.p[0];
+  c.inv_s = (float)(1.0 / M.p[1]);
+  c.v = (float)M.p[2];
+  c.ship_x = (float)M.p[3];
+  const double dn = M.kind == GEON_ALCUBIERRE ? M.alc_denom : 1.0;  // 2 tanh(R/s)
+  c.fnorm = (float)(1.0 / dn);
+  c.dfnorm = (float)(1.0 / (dn * M.p[1]));
+  c.cap_hi = (float)M.capture_r;
+  c.cap_lo = (float)(M.capture_r - (double)c.cap_hi);
+  c.esc_hi = (float)M.escape_r;
+  c.esc_lo = (float)(M.escape_r - (double)c.esc_hi);
+  c.cap_far = c.cap_hi * (1.0f + 0x1p-10f);
+  c.esc_far = c.esc_hi * (1.0f - 0x1p-10f);
+  c.r_near = 1.5f * c.two_m;
+  c.r_fast = std::fmax(c.two_m, c.cap_far);
+  c.h = (float)step;
+  c.hh = (float)half_step;
+  c.sixth = (float)sixth;
+  c.m2h = -2.0f * c.h;
+  c.m2sixth = -2.0f * c.sixth;
+  c.flat_r = std::isinf(M.alc_flat) ? INFINITY : std::nextafter((float)(M.p[0] + 9.5 * M.p[1] + 1e-3), INFINITY);
+  c.cap_steps = (float)max_steps;
+  return c;
+}
+
 TraceLaunch base_launch(geon_metric_t m, double step, int64_t max_steps) {
   TraceLaunch L;
   std::memset(&L, 0, sizeof L);
@@ -142,6 +174,7 @@ TraceLaunch base_launch(geon_metric_t m, double step, int64_t max_steps) {
   L.half_step = 0.5 * step;
   L.sixth = step / 6.0;
   L.max_steps = max_steps;
+  L.mx = mixed_consts(L.M, L.step, L.half_step, L.sixth, max_steps);
   L.band = g_band[m->desc.kind].load();
   L.mixed_flags = (g_reproject.load() ? MIXED_REPROJECT : 0) | (g_orbit.load() ? MIXED_ORBIT : 0) |
                   (g_nullfix.load() ? MIXED_NULLFIX : 0);

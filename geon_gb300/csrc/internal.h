@@ -74,8 +74,28 @@ enum : int { SRC_ARRAY = 0, SRC_CAMERA = 1, SRC_EQUATORIAL = 2, SRC_STATE = 3 };
 // steps), shaded by a later kernel; the trace kernel runs no FP64 sink code.
 enum : int { SINK_TRACE = 0, SINK_RENDER = 1, SINK_SHADOW = 2, SINK_STATE = 3 };
 
+// The constants of the mixed path's FP32 step (mixed_consts in capi.cu). A
+// kernel over one job reads them from its parameters, so they are constant-bank
+// operands: an FFMA with three register operands takes 1.5 issue cycles here,
+// with a constant for one of them 1 (measured 0.66 and 0.96 per cycle and SM
+// quarter), and they hold no registers.
+struct MixedConsts {
+  float m, two_m;                                // Schwarzschild
+  float b0sq;                                    // Morris-Thorne
+  float R, inv_s, v, ship_x, fnorm, dfnorm;      // Alcubierre: fnorm = 1/(2 tanh(R/s)), dfnorm = fnorm/s
+  float cap_hi, cap_lo, esc_hi, esc_lo;          // capture and escape radius as (high, low)
+  float cap_far, esc_far;                        // cap_hi (1 + 2^-10), esc_hi (1 - 2^-10)
+  float r_near;                                  // 3M (1.5 * 2M): inside it the horizon rules can apply
+  float r_fast;                                  // the larger of 2M and cap_far
+  float h, hh, sixth;                            // step, step / 2, step / 6
+  float m2h, m2sixth;                            // -2 h, -2 (h / 6)
+  float flat_r;                                  // Alcubierre: r_s from which the FP32 metric is flat
+  float cap_steps;                               // the step cap, for the early decision's budget test
+};
+
 struct TraceLaunch {
   MetricDesc M;
+  MixedConsts mx;
   CameraDesc cam;
   int64_t n;           // rays in the job
   double step;

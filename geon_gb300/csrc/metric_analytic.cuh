@@ -71,7 +71,7 @@ struct AMath<double> {
   static __device__ __forceinline__ void sincos(double x, double* s, double* c) { ::sincos(x, s, c); }
 };
 
-// Metric constants in the working precision.
+// Metric constants of the FP64 band steps (the FP32 step: MixedConsts).
 template <typename T>
 struct AConsts {
   T m, two_m;          // Schwarzschild
@@ -112,8 +112,8 @@ __device__ __forceinline__ void angle_add(T s0, T c0, T base, T d, T* s, T* c) {
 // l or x), x2 and x3 (y, z: Alcubierre only), the polar angle as th_base + dth
 // (Schwarzschild, Morris-Thorne: sin/cos of th_base are s0, c0) and the
 // momentum p. Unused arguments cost nothing (the compiler drops them).
-template <int K, typename T>
-__device__ __forceinline__ void rhs_stage(const AConsts<T>& C, T x1, T x2, T x3, T th_base, T dth, const T p[4],
+template <int K, typename T, class Consts>
+__device__ __forceinline__ void rhs_stage(const Consts& C, T x1, T x2, T x3, T th_base, T dth, const T p[4],
                                           T s0, T c0, T k[8]) {
   using Mt = AMath<T>;
   const T p0 = p[0], p1 = p[1], p2 = p[2], p3 = p[3];
@@ -179,13 +179,13 @@ template <int K, typename T>
 __device__ __forceinline__ void rhs_analytic(const AConsts<T>& C, const T xb[8], const T d[8], T s0, T c0,
                                              T k[8]) {
   const T p[4] = {xb[4] + d[4], xb[5] + d[5], xb[6] + d[6], xb[7] + d[7]};
-  rhs_stage<K, T>(C, xb[1] + d[1], xb[2] + d[2], xb[3] + d[3], xb[2], d[2], p, s0, c0, k);
+  rhs_stage<K, T, AConsts<T>>(C, xb[1] + d[1], xb[2] + d[2], xb[3] + d[3], xb[2], d[2], p, s0, c0, k);
 }
 
 // Null re-projection: solve g(p, p) = 0 for p^t at the point x, keeping the
 // spatial momentum and the sign of p^t. Returns the new p^t.
-template <int K, typename T>
-__device__ __forceinline__ T null_pt(const AConsts<T>& C, const T x[4], const T p[4], T s, T pt_now) {
+template <int K, typename T, class Consts>
+__device__ __forceinline__ T null_pt(const Consts& C, const T x[4], const T p[4], T s, T pt_now) {
   using Mt = AMath<T>;
   T pt;
   if (K == KIND_MINKOWSKI) {

@@ -150,47 +150,21 @@ __device__ __forceinline__ void serve_loop(const ServeJob* __restrict__ jobs, Se
     if (__ballot_sync(FULL, slot >= 0) == 0) break;
     if (slot >= 0) {
       const TraceLaunch& L = jobs[slot].L;
-      int inner = 0;
-      if (n + TRACE_INNER <= L.max_steps && st.flat_group(L)) {  // a whole group through flat space
-        n += TRACE_INNER;
-        inner = TRACE_INNER;
+      int t = TERM_NONE;
+      int64_t taken = 0;
+      n = group_steps(st, L, L.max_steps, n, t, taken);
+      if (t != TERM_NONE) {
+        double y[8];
+        st.to_double(y);
+        const int sink = jobs[slot].sink;
+        if (sink == SINK_RENDER) store_ray<K, SINK_RENDER>(L, ray, t, y, taken);
+        else if (sink == SINK_SHADOW) store_ray<K, SINK_SHADOW>(L, ray, t, y, taken);
+        else store_ray<K, SINK_TRACE>(L, ray, t, y, taken);
+        atomicAdd(&cnt.steps[slot], (unsigned long long)taken);
+        __threadfence();
+        atomicAdd(&cnt.done[slot], 1ull);
+        slot = -1;
       }
-#pragma unroll 1
-      for (; inner < TRACE_INNER; ++inner) {
-        int t = TERM_NONE;
-        long long taken = n;
-        if (n >= L.max_steps) {
-          t = TERM_DIVERGED;
-          taken = L.max_steps;
-        } else {
-          t = st.terminate(L);
-          if (t == TERM_NONE) {
-            const int r = st.step(L);
-            if (r == STEP_OK) {
-              ++n;
-            } else if (r == STEP_NONFINITE) {
-              t = TERM_DIVERGED;
-            } else {
-              t = TERM_CAPTURED;
-              taken = n + 1;
-            }
-          }
-        }
-        if (t != TERM_NONE) {
-          double y[8];
-          st.to_double(y);
-          const int sink = jobs[slot].sink;
-          if (sink == SINK_RENDER) store_ray<K, SINK_RENDER>(L, ray, t, y, taken);
-          else if (sink == SINK_SHADOW) store_ray<K, SINK_SHADOW>(L, ray, t, y, taken);
-          else store_ray<K, SINK_TRACE>(L, ray, t, y, taken);
-          atomicAdd(&cnt.steps[slot], (unsigned long long)taken);
-          __threadfence();
-          atomicAdd(&cnt.done[slot], 1ull);
-          slot = -1;
-          break;
-        }
-      }
-      if (slot >= 0) st.group_end(L);  // the ray survived a whole group of TRACE_INNER steps
     }
   }
   if (slot >= 0) {  // out of budget: park the ray for the next launch

@@ -130,7 +130,7 @@ struct AdaptiveStepper {
     }
     return STEP_NONFINITE;
   }
-  __device__ __forceinline__ bool flat_group(const TraceLaunch&) { return false; }
+  static constexpr bool FAST = false;
   __device__ __forceinline__ void group_end(const TraceLaunch&) {}
   __device__ __forceinline__ void check_null(const TraceLaunch&, const double*) {}
   __device__ __forceinline__ void finish(const TraceLaunch& L) {

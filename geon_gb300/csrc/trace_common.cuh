@@ -158,10 +158,12 @@ __device__ __forceinline__ int64_t group_steps(Stepper& st, const TraceLaunch& L
   const int left = left64 < (int64_t)TRACE_INNER ? (int)left64 : TRACE_INNER;
   int done = 0, extra = 0;
   t = TERM_NONE;
-  // a whole group through flat space at once (the same steps: see the steppers)
-  if (left == TRACE_INNER && st.flat_group(L)) done = TRACE_INNER;
 #pragma unroll 1
   for (; done < left; ++done) {
+    if constexpr (Stepper::FAST) {  // steps the stepper can take with fewer tests
+      done += st.fast_steps(L, left - done);
+      if (done >= left) break;
+    }
     t = st.terminate(L);
     if (t != TERM_NONE) break;
     const int r = st.step(L);
@@ -185,7 +187,9 @@ __device__ __forceinline__ int64_t group_steps(Stepper& st, const TraceLaunch& L
 // geodesic.rs:62-117 for every ray of the job, persistent over a work queue.
 // Stepper owns the ray state: load(y0), to_double(y), terminate(L), step(L)
 // returning STEP_OK (advanced), STEP_NONFINITE (state unchanged: Diverged) or
-// STEP_HORIZON (state unchanged: Captured after this step).
+// STEP_HORIZON (state unchanged: Captured after this step). Where Stepper::FAST,
+// fast_steps(L, left) takes some of the next `left` steps (their termination tests
+// answer "none" and they end STEP_OK, with the same result) and returns how many.
 template <class Stepper, int K, int SRC, int SINK>
 __device__ __forceinline__ void trace_loop(const TraceLaunch& L) {
   const unsigned FULL = 0xffffffffu;

@@ -70,8 +70,9 @@ struct Fp64Stepper {
     for (int i = 0; i < 8; ++i) y[i] = yn[i];
     return STEP_OK;
   }
-  __device__ __forceinline__ bool flat_group(const TraceLaunch& L) {
-    return K == KIND_ALCUBIERRE && alcubierre_flat_steps<TRACE_INNER>(L, y);
+  static constexpr bool FAST = K == KIND_ALCUBIERRE;
+  __device__ __forceinline__ int fast_steps(const TraceLaunch& L, int left) {
+    return K == KIND_ALCUBIERRE && left == TRACE_INNER && alcubierre_flat_steps<TRACE_INNER>(L, y) ? TRACE_INNER : 0;
   }
   __device__ __forceinline__ void group_end(const TraceLaunch&) {}
   __device__ __forceinline__ void check_null(const TraceLaunch&, const double*) {}
@@ -136,8 +137,9 @@ struct Fp64StepperAny {
     for (int i = 0; i < 8; ++i) y[i] = yn[i];
     return STEP_OK;
   }
-  __device__ __forceinline__ bool flat_group(const TraceLaunch& L) {
-    return kind == KIND_ALCUBIERRE && alcubierre_flat_steps<TRACE_INNER>(L, y);
+  static constexpr bool FAST = true;
+  __device__ __forceinline__ int fast_steps(const TraceLaunch& L, int left) {
+    return kind == KIND_ALCUBIERRE && left == TRACE_INNER && alcubierre_flat_steps<TRACE_INNER>(L, y) ? TRACE_INNER : 0;
   }
   __device__ __forceinline__ void group_end(const TraceLaunch&) {}
   __device__ __forceinline__ void check_null(const TraceLaunch&, const double*) {}

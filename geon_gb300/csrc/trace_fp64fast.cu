@@ -222,7 +222,7 @@ struct FastSchwStepper {
     for (int i = 0; i < 8; ++i) y[i] = yn[i];
     return STEP_OK;
   }
-  __device__ __forceinline__ bool flat_group(const TraceLaunch&) { return false; }
+  static constexpr bool FAST = false;
   __device__ __forceinline__ void group_end(const TraceLaunch&) {
     if (!PLANAR && !on_plane) dm::sincos_det(y[2], &sth, &cth);
   }

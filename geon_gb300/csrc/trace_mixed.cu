@@ -89,10 +89,12 @@ __device__ __forceinline__ bool ff_gt(float hi, float lo, float thi, float tlo) 
 // (Schwarzschild, Morris-Thorne) are turned into the frame of their own orbit
 // plane at load, stepped there on the equator, and turned back at the end;
 // FEAT_ORBIT_DYN: a per-ray flag says so (the serving kernel: camera rays).
+// FEAT_NO_TIME: the coordinate time of the final state is not read (a render's
+// states: neither the sky nor the residual depends on t), so planar steps leave it out.
 // FEAT_DECIDE: every ray is a bisection ray whose class settles early
 // (decided_k); FEAT_DECIDE_DYN: a per-ray flag says so (the serving kernel).
 enum : int { FEAT_BAND = 1, FEAT_REPROJECT = 2, FEAT_PLANAR = 4, FEAT_PLANAR_DYN = 8, FEAT_ORBIT = 16,
-             FEAT_ORBIT_DYN = 32, FEAT_DECIDE = 64, FEAT_DECIDE_DYN = 128 };
+             FEAT_ORBIT_DYN = 32, FEAT_DECIDE = 64, FEAT_DECIDE_DYN = 128, FEAT_NO_TIME = 256, FEAT_OWN = 512 };
 
 // Right-hand side on the equatorial plane: rhs_stage at sin theta = 1,
 // cos theta = 0, p^theta = 0, where its theta terms vanish (Gamma^th_phph =
@@ -100,7 +102,7 @@ enum : int { FEAT_BAND = 1, FEAT_REPROJECT = 2, FEAT_PLANAR = 4, FEAT_PLANAR_DYN
 // the same operations. The plane is invariant under the geodesic equation, so
 // a ray that starts in it stays in it. Schwarzschild (r) and Morris-Thorne (l).
 template <int K>
-__device__ __forceinline__ void rhs_planar(const AConsts<float>& C, float r, float p0, float p1, float p3,
+__device__ __forceinline__ void rhs_planar(const MixedConsts& C, float r, float p0, float p1, float p3,
                                            float* k4, float* k5, float* k7) {
   using Mt = AMath<float>;
   const float u = -2.0f * p1;  // shared by the Gamma^t_tr and Gamma^ph_rph terms
@@ -127,19 +129,18 @@ __device__ __forceinline__ void rhs_planar(const AConsts<float>& C, float r, flo
 template <int FEAT>
 struct MixedCore {
   float hi[8], lo[8];
-  AConsts<float> C;
-  float cap_hi, cap_lo, esc_hi, esc_lo;
-  float cap_far, esc_far;  // cap_hi (1 + 2^-10), esc_hi (1 - 2^-10)
-  float r_near;             // 3M (1.5 * 2M): inside it the horizon rules can apply
-  float h, hh, sixth;
-  float flat_r;             // Alcubierre: r_s from which the FP32 metric is flat
+  // FEAT_OWN: rays of several jobs pass through a lane, which keeps the
+  // constants of the job of its ray; otherwise they are the launch's.
+  MixedConsts own;
+  __device__ __forceinline__ const MixedConsts& consts(const TraceLaunch& L) const {
+    if constexpr ((FEAT & FEAT_OWN) != 0) return own;
+    else return L.mx;
+  }
   unsigned nsteps = 0;  // steps this ray has taken (counted where the early decision needs it)
-  bool ready = false;
   bool planar = (FEAT & FEAT_PLANAR) != 0;
   bool orbit = (FEAT & FEAT_ORBIT) != 0;
   bool decide = (FEAT & FEAT_DECIDE) != 0;
   bool nullray = true;  // the loaded state is null: the null re-projections apply
-  float cap_steps;  // the step cap (max_steps), for the early decision's budget test
   float oe1[3], oe2[3];  // orbit-plane frame (FEAT_ORBIT, FEAT_ORBIT_DYN)
   // rays of metric kind K can step in their orbit-plane frame
   template <int K>
@@ -169,20 +170,23 @@ struct MixedCore {
   }
 
   __device__ __forceinline__ void setup(const TraceLaunch& L) {
-    C.init(L.M);
-    cap_hi = __double2float_rn(L.M.capture_r);
-    cap_lo = __double2float_rn(L.M.capture_r - (double)cap_hi);
-    esc_hi = __double2float_rn(L.M.escape_r);
-    esc_lo = __double2float_rn(L.M.escape_r - (double)esc_hi);
-    cap_far = cap_hi * (1.0f + 0x1p-10f);
-    r_near = 1.5f * C.two_m;
-    esc_far = esc_hi * (1.0f - 0x1p-10f);
-    h = (float)L.step;
-    hh = (float)L.half_step;
-    sixth = (float)L.sixth;
-    cap_steps = (float)L.max_steps;
-    flat_r = isinf(L.M.alc_flat) ? INFINITY : __double2float_ru(L.M.p[0] + 9.5 * L.M.p[1] + 1e-3);
-    ready = true;
+    if constexpr ((FEAT & FEAT_OWN) != 0) own = L.mx;
+    if constexpr ((FEAT & FEAT_DECIDE) != 0) {
+      // Bisection rounds keep the step's constants in registers: with one warp
+      // per SM quarter the latency of a constant-bank read shows (6.5 against
+      // 5.9 ms). Converted from the FP64 values here (the same roundings as
+      // mixed_consts), because the compiler would read a plain copy again.
+      own.m = __double2float_rn(L.M.p[0]);
+      own.two_m = __double2float_rn(2.0 * L.M.p[0]);
+      own.h = __double2float_rn(L.step);
+      own.hh = __double2float_rn(L.half_step);
+      own.sixth = __double2float_rn(L.sixth);
+      own.esc_hi = __double2float_rn(L.M.escape_r);
+      own.cap_far = __double2float_rn(L.M.capture_r) * (1.0f + 0x1p-10f);
+      own.esc_far = own.esc_hi * (1.0f - 0x1p-10f);
+      own.r_near = 1.5f * own.two_m;
+      own.cap_steps = (float)L.max_steps;
+    }
   }
 
   __device__ __forceinline__ void load_state(const double y[8]) {
@@ -195,7 +199,7 @@ struct MixedCore {
 
   template <int K>
   __device__ __forceinline__ void load_k(const TraceLaunch& L, const double y0[8]) {
-    if (!ready) setup(L);
+    setup(L);
     nsteps = 0;
     if constexpr (any_orbit<K>()) {
       if (orbit) {
@@ -234,12 +238,12 @@ struct MixedCore {
   // left and is reported Captured now. The class is the one the full trace
   // would end with; steps_taken counts the steps actually taken.
   template <int K>
-  __device__ __forceinline__ int decided_k() const {
+  __device__ __forceinline__ int decided_k(const MixedConsts& Q) const {
     if (K == KIND_SCHWARZSCHILD) {
       if (hi[5] > 0.0f) {
-        if (hi[1] > 3.3f * C.m && (esc_hi - hi[1]) * 1.02f < (cap_steps - (float)nsteps - 2.0f) * h * hi[5])
+        if (hi[1] > 3.3f * Q.m && (Q.esc_hi - hi[1]) * 1.02f < (Q.cap_steps - (float)nsteps - 2.0f) * Q.h * hi[5])
           return TERM_ESCAPED;
-      } else if (hi[1] < 2.9f * C.m) {
+      } else if (hi[1] < 2.9f * Q.m) {
         return TERM_CAPTURED;
       }
     }
@@ -284,24 +288,25 @@ struct MixedCore {
     const bool on_plane = (any_orbit<K>() && orbit) ||
                           (K == KIND_SCHWARZSCHILD && (FEAT & (FEAT_PLANAR | FEAT_PLANAR_DYN)) != 0 &&
                            ((FEAT & FEAT_PLANAR) != 0 || planar));
-    if (on_plane) null_fix_planar<K>();
+    if (on_plane) null_fix_planar<K>(consts(L));
   }
 
   // Termination tests of the reference, evaluated on the compensated state.
   template <int K>
-  __device__ __forceinline__ int terminate_k(const TraceLaunch&) const {
+  __device__ __forceinline__ int terminate_k(const TraceLaunch& L) const {
+    const MixedConsts& Q = consts(L);
     if (K == KIND_SCHWARZSCHILD) {
       // Far from both radii the high word decides: |lo| <= ulp(hi)/2 = 2^-24
       // of hi, far inside the 2^-10 margins. (A non-finite r fails this test.)
-      if (hi[1] > cap_far && hi[1] < esc_far) {
+      if (hi[1] > Q.cap_far && hi[1] < Q.esc_far) {
         if constexpr ((FEAT & (FEAT_DECIDE | FEAT_DECIDE_DYN)) != 0) {
-          if (decide) return decided_k<K>();
+          if (decide) return decided_k<K>(Q);
         }
         return TERM_NONE;
       }
       if (!isfinite(hi[1])) return TERM_DIVERGED;
-      if (ff_gt(cap_hi, cap_lo, hi[1], lo[1])) return TERM_CAPTURED;
-      if (ff_gt(hi[1], lo[1], esc_hi, esc_lo)) return TERM_ESCAPED;
+      if (ff_gt(Q.cap_hi, Q.cap_lo, hi[1], lo[1])) return TERM_CAPTURED;
+      if (ff_gt(hi[1], lo[1], Q.esc_hi, Q.esc_lo)) return TERM_ESCAPED;
       return TERM_NONE;
     } else if (K == KIND_MORRIS_THORNE) {
       if (!isfinite(hi[1])) return TERM_DIVERGED;
@@ -324,11 +329,11 @@ struct MixedCore {
   //   f R = -(f p^t)^2 + (p^r)^2 + f (r p^phi)^2,  f = 1 - 2M/r;
   // Morris-Thorne: R = -(p^t)^2 + (p^l)^2 + (b0^2 + l^2) (p^phi)^2.
   template <int K>
-  __device__ __forceinline__ void null_fix_planar() {
+  __device__ __forceinline__ void null_fix_planar(const MixedConsts& Q) {
     const FF r = {hi[1], lo[1]}, pt = {hi[4], lo[4]}, pr = {hi[5], lo[5]}, pp = {hi[7], lo[7]};
     if (K == KIND_SCHWARZSCHILD) {
       const FF ir = ff_rcp(r);
-      const FF u = ff_mul({C.two_m, 0.0f}, ir);  // 2M / r
+      const FF u = ff_mul({Q.two_m, 0.0f}, ir);  // 2M / r
       const FF f = ff_add({1.0f, 0.0f}, {-u.h, -u.l});
       const FF E = ff_mul(f, pt);
       const FF w = ff_mul(r, pp);
@@ -338,7 +343,7 @@ struct MixedCore {
       const float d = (fR.h + fR.l) / (2.0f * f.h * E.h);
       if (isfinite(d)) two_sum_update(hi[4], lo[4], d);
     } else if (K == KIND_MORRIS_THORNE) {
-      const FF r2 = ff_add({C.b0sq, 0.0f}, ff_mul(r, r));
+      const FF r2 = ff_add({Q.b0sq, 0.0f}, ff_mul(r, r));
       const FF pt2 = ff_mul(pt, pt);
       const FF R = ff_add(ff_add(ff_mul(pr, pr), ff_mul(r2, ff_mul(pp, pp))), {-pt2.h, -pt2.l});
       const float d = (R.h + R.l) / (2.0f * pt.h);
@@ -354,8 +359,8 @@ struct MixedCore {
   // then reports it Escaped at r ~ 1e30 or Diverged). The ray is reported
   // Captured there instead. Elsewhere |increment / p^t| = 2 M h |p^r| / (r^2 f)
   // stays far below a quarter at any sensible step.
-  __device__ __forceinline__ bool unresolved_infall(float inc_pt) const {
-    return hi[5] < 0.0f && hi[1] < r_near && !(fabsf(inc_pt) < 0.25f * hi[4]);
+  __device__ __forceinline__ bool unresolved_infall(const MixedConsts& Q, float inc_pt) const {
+    return hi[5] < 0.0f && hi[1] < Q.r_near && !(fabsf(inc_pt) < 0.25f * hi[4]);
   }
 
   // Returns STEP_OK, STEP_NONFINITE (state unchanged) or STEP_HORIZON: an RK4
@@ -365,20 +370,21 @@ struct MixedCore {
   // step overflows or throws the ray to r ~ 1e30, reported Diverged or Escaped.)
   template <int K>
   __device__ __forceinline__ int step_fp32_k(const TraceLaunch& L) {
+    const MixedConsts& Q = consts(L);
     float s0 = 0.0f, c0 = 1.0f;
     if (K == KIND_SCHWARZSCHILD || K == KIND_MORRIS_THORNE) sincosf(hi[2], &s0, &c0);
     float k[8], acc[8], p[4];
     // stage 1 at the state (high words; the polar angle with its low word)
 #pragma unroll
     for (int i = 0; i < 4; ++i) p[i] = hi[4 + i];
-    rhs_stage<K, float>(C, hi[1], hi[2], hi[3], hi[2], lo[2], p, s0, c0, k);
+    rhs_stage<K, float, MixedConsts>(Q, hi[1], hi[2], hi[3], hi[2], lo[2], p, s0, c0, k);
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = k[i];
     // stages 2-4 at y + c h k
     float rmin = 0.0f;  // lowest stage radius (Schwarzschild horizon rule)
 #pragma unroll
     for (int st = 0; st < 3; ++st) {
-      const float c = st < 2 ? hh : h;
+      const float c = st < 2 ? Q.hh : Q.h;
 #pragma unroll
       for (int i = 0; i < 4; ++i) p[i] = __fmaf_rn(c, k[4 + i], hi[4 + i]);
       const float x1 = __fmaf_rn(c, k[1], hi[1]);
@@ -386,21 +392,21 @@ struct MixedCore {
       const float x3 = __fmaf_rn(c, k[3], hi[3]);
       const float dth = __fmaf_rn(c, k[2], lo[2]);
       rmin = st == 0 ? x1 : fminf(rmin, x1);
-      rhs_stage<K, float>(C, x1, x2, x3, hi[2], dth, p, s0, c0, k);
+      rhs_stage<K, float, MixedConsts>(Q, x1, x2, x3, hi[2], dth, p, s0, c0, k);
       if (st < 2) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i] = __fmaf_rn(2.0f, k[i], acc[i]);
       }
     }
-    if (K == KIND_SCHWARZSCHILD && !(rmin > C.two_m)) return STEP_HORIZON;
+    if (K == KIND_SCHWARZSCHILD && !(rmin > Q.two_m)) return STEP_HORIZON;
     bool finite = true;
     float inc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      inc[i] = sixth * (acc[i] + k[i]);
+      inc[i] = Q.sixth * (acc[i] + k[i]);
       finite &= isfinite(inc[i]);
     }
-    if (K == KIND_SCHWARZSCHILD && unresolved_infall(inc[4])) return STEP_HORIZON;
+    if (K == KIND_SCHWARZSCHILD && unresolved_infall(Q, inc[4])) return STEP_HORIZON;
     if (!finite) return STEP_NONFINITE;
     // Positions move monotonically in t and phi and stay far from 0 in r and
     // theta relative to one step, so Fast2Sum is exact for them (and for t = 0 or
@@ -418,7 +424,7 @@ struct MixedCore {
       if (K == KIND_SCHWARZSCHILD || K == KIND_MORRIS_THORNE) s = sinf(hi[2]);
       const float x[4] = {hi[0], hi[1], hi[2], hi[3]};
       const float p[4] = {hi[4], hi[5], hi[6], hi[7]};
-      const float pt = null_pt<K, float>(C, x, p, s, hi[4]);
+      const float pt = null_pt<K, float, MixedConsts>(Q, x, p, s, hi[4]);
       if (isfinite(pt)) {
         two_sum_update(hi[4], lo[4], (pt - hi[4]) - lo[4]);
       }
@@ -433,22 +439,23 @@ struct MixedCore {
   // horizon rule and compensated update as step_fp32.
   template <int K>
   __device__ __forceinline__ int step_fp32_planar_k(const TraceLaunch& L) {
+    const MixedConsts& Q = consts(L);
     float k1, k4, k5, k7;
     float p0 = hi[4], p1 = hi[5], p3 = hi[7];
-    rhs_planar<K>(C, hi[1], p0, p1, p3, &k4, &k5, &k7);
+    rhs_planar<K>(Q, hi[1], p0, p1, p3, &k4, &k5, &k7);
     k1 = p1;
     float a0 = p0, a1 = p1, a3 = p3, a4 = k4, a5 = k5, a7 = k7;
     float k0 = p0, k3 = p3;
     float rmin = 0.0f;
 #pragma unroll
     for (int st = 0; st < 3; ++st) {
-      const float c = st < 2 ? hh : h;
+      const float c = st < 2 ? Q.hh : Q.h;
       p0 = __fmaf_rn(c, k4, hi[4]);
       p1 = __fmaf_rn(c, k5, hi[5]);
       p3 = __fmaf_rn(c, k7, hi[7]);
       const float r = __fmaf_rn(c, k1, hi[1]);
       rmin = st == 0 ? r : fminf(rmin, r);
-      rhs_planar<K>(C, r, p0, p1, p3, &k4, &k5, &k7);
+      rhs_planar<K>(Q, r, p0, p1, p3, &k4, &k5, &k7);
       k0 = p0; k1 = p1; k3 = p3;
       if (st < 2) {
         a0 = __fmaf_rn(2.0f, k0, a0);
@@ -459,8 +466,8 @@ struct MixedCore {
         a7 = __fmaf_rn(2.0f, k7, a7);
       }
     }
-    const float i0 = sixth * (a0 + k0), i1 = sixth * (a1 + k1), i3 = sixth * (a3 + k3);
-    const float i4 = sixth * (a4 + k4), i5 = sixth * (a5 + k5), i7 = sixth * (a7 + k7);
+    const float i0 = Q.sixth * (a0 + k0), i1 = Q.sixth * (a1 + k1), i3 = Q.sixth * (a3 + k3);
+    const float i4 = Q.sixth * (a4 + k4), i5 = Q.sixth * (a5 + k5), i7 = Q.sixth * (a7 + k7);
     // The horizon rules (a stage at or inside 2M; an unresolved infall, which
     // needs r < 3M) apply only when a stage or the ray is within 3M (or a
     // stage radius is not a number), and the NaN guard on the momenta only
@@ -471,10 +478,10 @@ struct MixedCore {
     // momentum increment; positions that nothing reads, t and phi for the
     // shadow sink, are then left out by the compiler.)
     const bool finite = isfinite(i4) && isfinite(i5) && isfinite(i7);
-    const bool near = K == KIND_SCHWARZSCHILD && (!(rmin > r_near) || hi[1] < r_near);
+    const bool near = K == KIND_SCHWARZSCHILD && (!(rmin > Q.r_near) || hi[1] < Q.r_near);
     if (near || !finite) {
-      if (K == KIND_SCHWARZSCHILD && !(rmin > C.two_m)) return STEP_HORIZON;
-      if (K == KIND_SCHWARZSCHILD && near && unresolved_infall(i4)) return STEP_HORIZON;
+      if (K == KIND_SCHWARZSCHILD && !(rmin > Q.two_m)) return STEP_HORIZON;
+      if (K == KIND_SCHWARZSCHILD && near && unresolved_infall(Q, i4)) return STEP_HORIZON;
       if (!finite) return STEP_NONFINITE;
     }
     fast_two_sum_update(hi[0], lo[0], i0);
@@ -492,7 +499,7 @@ struct MixedCore {
     if ((FEAT & FEAT_REPROJECT) && (L.mixed_flags & MIXED_REPROJECT) && nullray) {
       const float x[4] = {hi[0], hi[1], hi[2], hi[3]};
       const float p[4] = {hi[4], hi[5], 0.0f, hi[7]};
-      const float pt = null_pt<K, float>(C, x, p, 1.0f, hi[4]);
+      const float pt = null_pt<K, float, MixedConsts>(Q, x, p, 1.0f, hi[4]);
       if (isfinite(pt)) two_sum_update(hi[4], lo[4], (pt - hi[4]) - lo[4]);
     }
     return STEP_OK;
@@ -513,36 +520,147 @@ struct MixedCore {
   // (512 x 384 Alcubierre with Morris-Thorne in one launch: 66.8 -> 21.0 ms).
   template <int K, int N>
   __device__ __forceinline__ bool flat_group_k(const TraceLaunch& L) {
-    if constexpr (K != KIND_ALCUBIERRE || (FEAT & (FEAT_BAND | FEAT_REPROJECT)) != 0) {
+    const MixedConsts& Q = consts(L);
+    const float X = hi[1] - Q.ship_x;
+    const float yz = __fmaf_rn(hi[2], hi[2], hi[3] * hi[3]);
+    const float path = (1.001f * N) * Q.h * (fabsf(hi[5]) + fabsf(hi[6]) + fabsf(hi[7]));
+    const float inner = Q.flat_r + path, outer = 999.0f - path;
+    if (!(__fmaf_rn(X, X, yz) > 1.001f * (inner * inner)) || !(outer > 0.0f) ||
+        !(__fmaf_rn(hi[1], hi[1], yz) < outer * outer))
       return false;
+    if (!(Q.h > 0.0f) || !(fabsf(hi[4]) < 1e10f) || !(fabsf(hi[0]) < 1e10f) || !(Q.h < 1e6f)) return false;
+    float mh[4], ml[4];
+    bool same = true;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      mh[i] = hi[4 + i];
+      ml[i] = lo[4 + i];
+      two_sum_update(mh[i], ml[i], 0.0f);
+      same &= mh[i] == hi[4 + i];
+    }
+    if (!same) return false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      lo[4 + i] = ml[i];
+      const float p = hi[4 + i];
+      const float inc = Q.sixth * (__fmaf_rn(2.0f, p, __fmaf_rn(2.0f, p, p)) + p);
+#pragma unroll
+      for (int q = 0; q < N; ++q) two_sum_update(hi[i], lo[i], inc);
+    }
+    return true;
+  }
+
+  // Steps of a ray on its plane while nothing but the step itself has to be
+  // done: the radius and every stage radius above r_fast (2M and the capture
+  // radius with its margin) and, inside 3M, the infall resolved; the radius below
+  // the escape radius with its margin; every momentum increment finite. There
+  // the termination test answers "none" and no horizon rule applies, so one
+  // combined test and branch replace those of terminate_k and
+  // step_fp32_planar_k; a step that fails it is left to those (the state is not
+  // touched). The arithmetic is step_fp32_planar_k's with the factor -2 of the
+  // p^t and p^phi derivatives moved into the constants they meet (scaling by a
+  // power of two is exact), which saves a multiplication per right-hand side;
+  // the same bits.
+  template <int K>
+  __device__ __forceinline__ int planar_steps_k(const MixedConsts& Q, int left) {
+    constexpr bool S = K == KIND_SCHWARZSCHILD;
+    constexpr bool TIME = (FEAT & FEAT_NO_TIME) == 0;
+    if (!S && !TIME) fast_two_sum_update(hi[4], lo[4], 0.0f);  // p^t: a zero increment each step
+    int done = 0;
+#pragma unroll 1
+    for (; done < left; ++done) {
+      float w4 = 0.0f, k5, w7;  // k4 = -2 w4, k7 = -2 w7
+      float p0 = hi[4], p1 = hi[5], p3 = hi[7], r = hi[1];
+      planar_rhs<K>(Q, r, p0, p1, p3, w4, k5, w7);
+      float a0 = p0, a1 = p1, a3 = p3, a4 = w4, a5 = k5, a7 = w7;
+      float rs[4] = {r, r, r, r};
+#pragma unroll
+      for (int st = 0; st < 3; ++st) {
+        const float c = st < 2 ? Q.hh : Q.h, m2c = st < 2 ? -Q.h : Q.m2h;  // -2 hh = -h
+        r = __fmaf_rn(c, p1, hi[1]);
+        if (S || TIME) p0 = __fmaf_rn(m2c, w4, hi[4]);
+        p1 = __fmaf_rn(c, k5, hi[5]);
+        p3 = __fmaf_rn(m2c, w7, hi[7]);
+        rs[st + 1] = r;
+        planar_rhs<K>(Q, r, p0, p1, p3, w4, k5, w7);
+        if (st < 2) {
+          if (TIME) a0 = __fmaf_rn(2.0f, p0, a0);
+          a1 = __fmaf_rn(2.0f, p1, a1);
+          a3 = __fmaf_rn(2.0f, p3, a3);
+          if (S) a4 = __fmaf_rn(2.0f, w4, a4);
+          a5 = __fmaf_rn(2.0f, k5, a5);
+          a7 = __fmaf_rn(2.0f, w7, a7);
+        }
+      }
+      const float i4 = S ? Q.m2sixth * (a4 + w4) : 0.0f;
+      const float i5 = Q.sixth * (a5 + k5), i7 = Q.m2sixth * (a7 + w7);
+      bool ok;
+      if (S) {
+        const float rmin = fminf(fminf(rs[0], rs[1]), fminf(rs[2], rs[3]));
+        ok = (max_nan(fabsf(i4), fabsf(i5), fabsf(i7)) < INFINITY) & (rmin > Q.r_fast) & (hi[1] < Q.esc_far) &
+             ((rmin > Q.r_near) | (fabsf(i4) < 0.25f * hi[4]));
+      } else {
+        ok = (fabsf(i5) < INFINITY) & (fabsf(i7) < INFINITY) & (fabsf(hi[1]) < 999.0f);
+      }
+      if ((FEAT & FEAT_DECIDE_DYN) != 0) ok = ok & !(decide & (hi[5] > 0.0f ? hi[1] > 3.3f * Q.m : hi[1] < 2.9f * Q.m));
+      if (!ok) break;
+      if (TIME) fast_two_sum_update(hi[0], lo[0], Q.sixth * (a0 + p0));
+      fast_two_sum_update(hi[1], lo[1], Q.sixth * (a1 + p1));
+      fast_two_sum_update(hi[3], lo[3], Q.sixth * (a3 + p3));
+      if (S || TIME) fast_two_sum_update(hi[4], lo[4], i4);
+      two_sum_update(hi[5], lo[5], i5);
+      fast_two_sum_update(hi[7], lo[7], i7);
+      count_step();
+    }
+    return done;
+  }
+  // the largest of three, NaN if one is NaN
+  static __device__ __forceinline__ float max_nan(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+  }
+
+  // rhs_planar with k4 = -2 w4 and k7 = -2 w7 (exactly).
+  template <int K>
+  __device__ __forceinline__ void planar_rhs(const MixedConsts& Q, float r, float p0, float p1, float p3, float& w4, float& k5, float& w7) {
+    using Mt = AMath<float>;
+    if (K == KIND_MORRIS_THORNE) {
+      const float q = Mt::div(r, Mt::fma(r, r, Q.b0sq));
+      k5 = r * (p3 * p3);
+      w7 = (p1 * q) * p3;
+      return;
+    }
+    const float rm = r - Q.two_m;
+    const float iD = Mt::rcp(r * rm);
+    const float gtr = Q.m * iD;
+    const float ir = rm * iD;
+    const float E = (rm * ir) * p0;
+    w4 = (p1 * gtr) * p0;
+    k5 = Mt::fma(gtr, Mt::fma(-E, E, p1 * p1), rm * (p3 * p3));
+    w7 = (p1 * ir) * p3;
+  }
+  // Rays of kind K have fast steps. Not the bisection rounds: a ray of theirs
+  // is decided by tests between its steps, and with one warp per SM quarter a
+  // round takes as long as its slowest ray's chain of steps, which the combined
+  // test lengthens (64 brackets of 40 halvings: 7.3 ms with it, 5.9 without).
+  template <int K>
+  static constexpr bool any_fast() {
+    return K == KIND_ALCUBIERRE ? (FEAT & (FEAT_BAND | FEAT_REPROJECT)) == 0
+                                : (FEAT & (FEAT_BAND | FEAT_REPROJECT | FEAT_DECIDE)) == 0 &&
+                                      (any_orbit<K>() || (K == KIND_SCHWARZSCHILD &&
+                                                          (FEAT & (FEAT_PLANAR | FEAT_PLANAR_DYN)) != 0));
+  }
+  template <int K>
+  __device__ __forceinline__ int fast_steps_k(const TraceLaunch& L, int left) {
+    if constexpr (!any_fast<K>()) {
+      return 0;
+    } else if constexpr (K == KIND_ALCUBIERRE) {
+      return left == TRACE_INNER && flat_group_k<K, TRACE_INNER>(L) ? TRACE_INNER : 0;
     } else {
-      const float X = hi[1] - C.ship_x;
-      const float yz = __fmaf_rn(hi[2], hi[2], hi[3] * hi[3]);
-      const float path = (1.001f * N) * h * (fabsf(hi[5]) + fabsf(hi[6]) + fabsf(hi[7]));
-      const float inner = flat_r + path, outer = 999.0f - path;
-      if (!(__fmaf_rn(X, X, yz) > 1.001f * (inner * inner)) || !(outer > 0.0f) ||
-          !(__fmaf_rn(hi[1], hi[1], yz) < outer * outer))
-        return false;
-      if (!(h > 0.0f) || !(fabsf(hi[4]) < 1e10f) || !(fabsf(hi[0]) < 1e10f) || !(h < 1e6f)) return false;
-      float mh[4], ml[4];
-      bool same = true;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        mh[i] = hi[4 + i];
-        ml[i] = lo[4 + i];
-        two_sum_update(mh[i], ml[i], 0.0f);
-        same &= mh[i] == hi[4 + i];
-      }
-      if (!same) return false;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        lo[4 + i] = ml[i];
-        const float p = hi[4 + i];
-        const float inc = sixth * (__fmaf_rn(2.0f, p, __fmaf_rn(2.0f, p, p)) + p);
-#pragma unroll
-        for (int q = 0; q < N; ++q) two_sum_update(hi[i], lo[i], inc);
-      }
-      return true;
+      const bool on_plane = (any_orbit<K>() && orbit) || (FEAT & FEAT_PLANAR) != 0 ||
+                            ((FEAT & FEAT_PLANAR_DYN) != 0 && planar);
+      return on_plane ? planar_steps_k<K>(consts(L), left) : 0;
     }
   }
 
@@ -636,8 +754,9 @@ struct MixedStepper : MixedCore<FEAT> {
   __device__ __forceinline__ void to_double(double out[8]) const { this->template to_double_k<K>(out); }
   __device__ __forceinline__ int terminate(const TraceLaunch& L) const { return this->template terminate_k<K>(L); }
   __device__ __forceinline__ int step(const TraceLaunch& L) { return this->template step_k<K>(L); }
-  __device__ __forceinline__ bool flat_group(const TraceLaunch& L) {
-    return this->template flat_group_k<K, TRACE_INNER>(L);
+  static constexpr bool FAST = MixedCore<FEAT>::template any_fast<K>();
+  __device__ __forceinline__ int fast_steps(const TraceLaunch& L, int left) {
+    return this->template fast_steps_k<K>(L, left);
   }
   __device__ __forceinline__ void group_end(const TraceLaunch& L) { this->template group_end_k<K>(L); }
   __device__ __forceinline__ void check_null(const TraceLaunch& L, const double y0[8]) {
@@ -692,8 +811,9 @@ struct MixedStepperAny : MixedCore<FEAT> {
   __device__ __forceinline__ int step(const TraceLaunch& L) {
     return on_kind([&](auto k) { return this->template step_k<decltype(k)::value>(L); });
   }
-  __device__ __forceinline__ bool flat_group(const TraceLaunch& L) {
-    return on_kind([&](auto k) { return this->template flat_group_k<decltype(k)::value, TRACE_INNER>(L); });
+  static constexpr bool FAST = true;
+  __device__ __forceinline__ int fast_steps(const TraceLaunch& L, int left) {
+    return on_kind([&](auto k) { return this->template fast_steps_k<decltype(k)::value>(L, left); });
   }
   __device__ __forceinline__ void group_end(const TraceLaunch& L) {
     on_kind([&](auto k) { this->template group_end_k<decltype(k)::value>(L); });
@@ -704,10 +824,17 @@ struct MixedStepperAny : MixedCore<FEAT> {
 };
 
 // MINB is the register cap chosen by the autotuner: __launch_bounds__(BLOCK,
-// MINB) asks the compiler to fit MINB blocks per SM (1: no cap, 63 registers
-// and 8 blocks of 128 for the planar equatorial step, 72 and 7 for the camera
+// MINB) asks the compiler to fit MINB blocks per SM (1: no cap, 56 registers
+// and 9 blocks of 128 for the planar equatorial step, 59 and 8 for the camera
 // step; 8 blocks of 128: <= 64 registers; 10: <= 51), trading registers (and
-// spills) for resident warps. BLOCK is the block size (128 except for the
+// spills) for resident warps. Measured with the combined test and the
+// constant-bank constants, before and after: the 2^20-ray sweep 274 -> 268 ms
+// (cap 10), a 960 x 540 frame with 4 samples per pixel 29.4 -> 26.9 ms. What
+// bounds the step is not its instruction count any more (144 -> 139 of them,
+// and 126 in a version that tested only every fourth step ran no faster) but
+// the FP32 pipe with its register reads: 110 FP32 operations in ~158 cycles per
+// SM quarter; FFMA with three registers issues at 0.66 per cycle, and a mix of
+// FFMA, FADD and FMUL at 0.79. BLOCK is the block size (128 except for the
 // equatorial shadow kernel, whose autotuner also tries 64 and 256).
 template <int K, int SRC, int SINK, int MINB, int FEAT, int BLOCK = TRACE_BLOCK>
 __global__ void __launch_bounds__(BLOCK, MINB) trace_mixed_kernel(const TraceLaunch L) {
@@ -744,10 +871,11 @@ static cudaError_t launch_mst(const TraceLaunch& L, cudaStream_t s) {
     // orbit-plane frame (the default for camera rays and ray arrays of the
     // spherically symmetric metrics; equatorial rays already step on their plane)
     if (feat == 0 && (L.mixed_flags & MIXED_ORBIT)) {
+      constexpr int F = FEAT_ORBIT | (SINK == SINK_STATE ? FEAT_NO_TIME : 0);
       switch (L.variant % 3) {
-        case 1: return launch_mst_v<K, SRC, SINK, 8, FEAT_ORBIT>(L, s);
-        case 2: return launch_mst_v<K, SRC, SINK, 10, FEAT_ORBIT>(L, s);
-        default: return launch_mst_v<K, SRC, SINK, 1, FEAT_ORBIT>(L, s);
+        case 1: return launch_mst_v<K, SRC, SINK, 8, F>(L, s);
+        case 2: return launch_mst_v<K, SRC, SINK, 10, F>(L, s);
+        default: return launch_mst_v<K, SRC, SINK, 1, F>(L, s);
       }
     }
   }
@@ -757,7 +885,7 @@ static cudaError_t launch_mst(const TraceLaunch& L, cudaStream_t s) {
     case FEAT_BAND | FEAT_REPROJECT: return launch_mst_v<K, SRC, SINK, 1, FEAT_BAND | FEAT_REPROJECT>(L, s);
   }
   if constexpr (SRC == SRC_EQUATORIAL && SINK == SINK_SHADOW) {
-    if (L.decide) return launch_mst_v<K, SRC, SINK, 1, FEAT_DECIDE>(L, s);  // bisection rounds
+    if (L.decide) return launch_mst_v<K, SRC, SINK, 1, FEAT_DECIDE | FEAT_OWN>(L, s);  // bisection rounds
     // variant = register cap + 3 * block size (128, 64, 256); the same caps in
     // registers per thread (64, 51) at every block size
     switch (L.variant) {
@@ -788,7 +916,7 @@ static cudaError_t launch_mst(const TraceLaunch& L, cudaStream_t s) {
 // prepare and shade kernels.
 template <int KMASK>
 __global__ void __launch_bounds__(TRACE_BLOCK) trace_multi_mixed_kernel(const TraceLaunch* jobs, const MultiDesc D) {
-  trace_loop_multi<MixedStepperAny<FEAT_ORBIT_DYN, KMASK>, SRC_STATE, SINK_STATE>(jobs, D);
+  trace_loop_multi<MixedStepperAny<FEAT_OWN | FEAT_ORBIT_DYN | FEAT_NO_TIME, KMASK>, SRC_STATE, SINK_STATE>(jobs, D);
 }
 
 template <int KMASK>
@@ -832,8 +960,8 @@ cudaError_t launch_trace_multi_mixed(const TraceLaunch* jobs, const MultiDesc& D
 template <int K>
 __global__ void __launch_bounds__(TRACE_BLOCK, 7) serve_mixed_kernel(const ServeJob* jobs, ServeCounters cnt,
                                                                      ServeClass* cl, const unsigned* epoch, int budget) {
-  constexpr int F = K == KIND_SCHWARZSCHILD ? (FEAT_PLANAR_DYN | FEAT_ORBIT_DYN | FEAT_DECIDE_DYN)
-                    : K == KIND_MORRIS_THORNE ? FEAT_ORBIT_DYN : 0;
+  constexpr int F = FEAT_OWN | (K == KIND_SCHWARZSCHILD ? (FEAT_PLANAR_DYN | FEAT_ORBIT_DYN | FEAT_DECIDE_DYN)
+                                : K == KIND_MORRIS_THORNE ? FEAT_ORBIT_DYN : 0);
   serve_loop<MixedStepper<K, F>, K>(jobs, cnt, cl, epoch, budget);
 }
 

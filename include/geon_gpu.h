@@ -280,7 +280,8 @@ void geon_set_persistent_reserve_f(double blocks_per_sm);
  * camera rays and ray arrays, 1: equatorial shadow rays). Register cap c: 0 =
  * none, 1 = at most 64 registers per thread, 2 = at most 51. Source 0 takes
  * variant = c (blocks of 128 threads); source 1 takes variant = c + 3 b with
- * block size b: 0 = 128, 1 = 64, 2 = 256 threads. geon_autotune_mixed times
+ * block size b: 0 = 128, 1 = 64, 2 = 256 threads. Defaults: 0, for the
+ * Schwarzschild equatorial source 2. geon_autotune_mixed times
  * every variant on calibration jobs of this metric (n_rays rays - 0 picks four
  * per lane of the widest grid - at most max_steps each; the equatorial job only
  * for Schwarzschild), selects the fastest per source and writes ray-steps/s to
