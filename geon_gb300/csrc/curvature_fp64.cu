@@ -33,6 +33,8 @@
 
 namespace geon {
 
+#include "curvature_sparse.cuh"
+
 constexpr int CURV_PPB = 16;       // points per block
 constexpr int CURV_THREADS = 128;
 static_assert(CURV_PPB <= 32 && CURV_THREADS >= 32 + CURV_PPB, "the tetrads run on the second warp");
@@ -420,10 +422,419 @@ curvature_kernel(const MetricDesc M, int what, const double* __restrict__ xs, in
   }
 }
 
+// ---------------------------------------------------------------------------
+// One thread per point (Alcubierre, Morris-Thorne, Schwarzschild).
+//
+// The cooperative kernel above spends most of its FP64 operations on structural
+// zeros (dense Riemann sums, dense Gram-Schmidt) and leaves lanes idle in its
+// per-point parts. Here a thread evaluates a whole point with the generated
+// sparse code of curvature_sparse.cuh: the metric values of the stencil into
+// shared memory (one column per thread), the distinct nonzero symbols slot by
+// slot, their differences, the sparse Ricci tensor, and the vectors of the point
+// one after another. Terms that are structurally zero, or the difference of two
+// equal values, are left out, so finite results have the dense code's bits up
+// to the sign of a zero; a point with a singular metric or a non-finite symbol
+// goes through the dense sums (dense_ricci), which treat it as before.
+// Divisions and square roots run in the integer pipes (softfp.cuh), and so do
+// the tests and the conversion of the random directions. Still bound by the FP64
+// pipe, with about 4400 instead of 10400 FP64 operations per Alcubierre point
+// and 32 of 32 lanes instead of 27: 128^3 points with 16 vectors 43.4 -> 18.2 ms,
+// 32736 Morris-Thorne points 518 -> 170 us, 10^5 Schwarzschild scalars 486 -> 90 us.
+// ---------------------------------------------------------------------------
+constexpr int POINT_THREADS = 64;
+
+// Ricci tensor of one point by the dense sums of curvature.rs:48-85.
+template <int K>
+__device__ __noinline__ void dense_ricci(const MetricDesc& M, const double x[4], double* ric, int* flags) {
+  using ST = Stencil<K>;
+  double G[ST::slots][64];
+  for (int sl = 0; sl < ST::slots; ++sl) {
+    double xs[4];
+    ST::slot_point(x, sl, xs);
+    if (!metric_christoffel<K>(M, xs, G[sl])) atomicOr(flags, 1);
+  }
+  const double inv_2h = 1.0 / (2.0 * FD_H);
+  for (int mu = 0; mu < 4; ++mu)
+    for (int nu = 0; nu < 4; ++nu) {
+      double s = 0.0;
+      for (int al = 0; al < 4; ++al) {  // R^al_{mu al nu}
+        const double* g0 = G[0];
+        const double term1 = (G[ST::slot_for(al, 0)][16 * al + 4 * nu + mu] - G[ST::slot_for(al, 1)][16 * al + 4 * nu + mu]) * inv_2h;
+        const double term2 = (G[ST::slot_for(nu, 0)][16 * al + 4 * al + mu] - G[ST::slot_for(nu, 1)][16 * al + 4 * al + mu]) * inv_2h;
+        double term3 = 0.0, term4 = 0.0;
+        for (int la = 0; la < 4; ++la) {
+          term3 += g0[16 * al + 4 * al + la] * g0[16 * la + 4 * nu + mu];
+          term4 += g0[16 * al + 4 * nu + la] * g0[16 * la + 4 * al + mu];
+        }
+        s += term1 - term2 + term3 - term4;
+      }
+      ric[4 * mu + nu] = s;
+    }
+}
+
+// What the point kernel needs of a metric:
+//   NV doubles of metric values per thread, ND differences per axis;
+//   values(M, x, v): the metric values of every stencil position, v[q * THREADS];
+//   symbols(M, x, v, slot, c): the distinct symbols of a slot;
+//   ricci(c, d, ric), metric(M, x, v, g, gi): the nonzero entries of g and g^-1;
+//   diff_place(i): the place of symbol i among the stored differences, or -1;
+//   GMASK: the entries of g that are not zero.
+template <int K>
+struct PointMetric;
+
+template <>
+struct PointMetric<KIND_ALCUBIERRE> {
+  using ST = Stencil<KIND_ALCUBIERRE>;
+  static constexpr int NG = ALCUBIERRE_GAMMAS, ND = ALCUBIERRE_DIFFS, GMASK = 0x8433;
+  // the metric function f at the 31 positions; while they are formed, the
+  // squares of the 7 shifted coordinates per axis lie where the differences will
+  static constexpr int NV = ST::positions;
+  static_assert(21 <= 3 * ND, "the squares fit into the store of the differences");
+  __device__ static __forceinline__ void values(const MetricDesc& M, const double x[4], double* v, double* store) {
+    // shifts of one axis: 0, +h, -h, then (+h) +h, (+h) -h, (-h) +h, (-h) -h
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double c = x[a + 1], p = c + FD_H, m = c - FD_H;
+      const double s[7] = {c, p, m, p + FD_H, p - FD_H, m + FD_H, m - FD_H};
+#pragma unroll
+      for (int i = 0; i < 7; ++i) {
+        const double d = a == 0 ? s[i] - M.p[3] : s[i];
+        store[(7 * a + i) * POINT_THREADS] = d * d;
+      }
+    }
+    const double R = M.p[0], th = M.p[1];
+#pragma unroll 1
+    for (int q = 0; q < ST::positions; ++q) {  // Stencil::position's numbering
+      int sx = 0, sy = 0, sz = 0;
+      if (q >= 1 && q < 7) {
+        const int a = (q - 1) >> 1, i = 1 + ((q - 1) & 1);
+        sx = a == 0 ? i : 0, sy = a == 1 ? i : 0, sz = a == 2 ? i : 0;
+      } else if (q >= 7 && q < 19) {
+        const int a = (q - 7) >> 2, i = 3 + ((q - 7) & 3);
+        sx = a == 0 ? i : 0, sy = a == 1 ? i : 0, sz = a == 2 ? i : 0;
+      } else if (q >= 19) {
+        const int pr = (q - 19) >> 2, i = 1 + (((q - 19) >> 1) & 1), j = 1 + ((q - 19) & 1);
+        sx = pr < 2 ? i : 0, sy = pr == 0 ? j : (pr == 2 ? i : 0), sz = pr >= 1 ? j : 0;
+      }
+      const double rs = sf::root(store[sx * POINT_THREADS] + store[(7 + sy) * POINT_THREADS] +
+                                 store[(14 + sz) * POINT_THREADS]);
+      const double t_plus = dm::tanh_det(sf::div(rs + R, th));
+      const double t_minus = dm::tanh_det(sf::div(rs - R, th));
+      v[q * POINT_THREADS] = sf::div(t_plus - t_minus, M.alc_denom);
+    }
+  }
+  __device__ static __forceinline__ void entry(const MetricDesc& M, double f, double* g00, double* g01) {
+    const double v = M.p[2];
+    *g00 = -1.0 + v * v * f * f;
+    *g01 = -v * f;
+  }
+  __device__ static __forceinline__ bool symbols(const MetricDesc& M, const double*, const double* v, int slot, double* c) {
+    double gv[14];
+#pragma unroll
+    for (int tag = 0; tag < 7; ++tag)
+      entry(M, v[ST::input_position(slot, tag) * POINT_THREADS], gv + 2 * tag, gv + 2 * tag + 1);
+    return alcubierre_gammas(gv, c);
+  }
+  template <class D>
+  __device__ static __forceinline__ void ricci(const double* c, D d, double* ric) { alcubierre_ricci(c, d, ric); }
+  __device__ static constexpr int diff_place(int i) { return alcubierre_diff_place(i); }
+  __device__ static __forceinline__ void metric(const MetricDesc& M, const double*, const double* v, double* g, double* gi) {
+    double gv[2];
+    entry(M, v[0], gv, gv + 1);
+    g[0] = gv[0]; g[1] = gv[1]; g[4] = gv[1]; g[5] = 1.0; g[10] = 1.0; g[15] = 1.0;
+    alcubierre_inverse(gv, gi);
+  }
+};
+
+template <>
+struct PointMetric<KIND_MORRIS_THORNE> {
+  using ST = Stencil<KIND_MORRIS_THORNE>;
+  static constexpr int NG = MORRIS_THORNE_GAMMAS, ND = MORRIS_THORNE_DIFFS, GMASK = 0x8421;
+  // r^2 = b0^2 + l^2 at the 7 shifted l and sin(theta) at the 7 shifted theta
+  static constexpr int NV = 14;
+  __device__ static __forceinline__ void values(const MetricDesc& M, const double x[4], double* v, double*) {
+    const double b0 = M.p[0];
+#pragma unroll 1
+    for (int i = 0; i < 7; ++i) {
+      const int s1 = i < 3 ? i : 1 + ((i - 3) >> 1), s2 = i < 3 ? 0 : 1 + ((i - 3) & 1);
+      double l = x[1], th = x[2];
+      if (s1) l = ST::shift(l, s1 - 1), th = ST::shift(th, s1 - 1);
+      if (s2) l = ST::shift(l, s2 - 1), th = ST::shift(th, s2 - 1);
+      v[i * POINT_THREADS] = b0 * b0 + l * l;
+      double s, c;
+      dm::sincos_det(th, &s, &c);
+      v[(7 + i) * POINT_THREADS] = s;
+    }
+  }
+  // g_thth and g_phph at shift i of l and shift j of theta (mt_g22_g33)
+  __device__ static __forceinline__ void entry(const double* v, int i, int j, double* g) {
+    const double r2 = v[i * POINT_THREADS], s = v[(7 + j) * POINT_THREADS];
+    g[0] = r2;
+    g[1] = r2 * s * s;
+  }
+  __device__ static __forceinline__ bool symbols(const MetricDesc&, const double*, const double* v, int slot, double* c) {
+    // slot: 0 the point, 1 + m its shift along l, 3 + m along theta; tag 1 + n along l, 3 + n along theta
+    const int li = slot == 1 || slot == 2 ? slot : 0, ti = slot >= 3 ? slot - 2 : 0;
+    double gv[10];
+    entry(v, li, ti, gv);
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      entry(v, li ? 1 + 2 * li + n : 1 + n, ti, gv + 2 + 2 * n);
+      entry(v, li, ti ? 1 + 2 * ti + n : 1 + n, gv + 6 + 2 * n);
+    }
+    return morris_thorne_gammas(gv, c);
+  }
+  template <class D>
+  __device__ static __forceinline__ void ricci(const double* c, D d, double* ric) { morris_thorne_ricci(c, d, ric); }
+  __device__ static constexpr int diff_place(int i) { return morris_thorne_diff_place(i); }
+  __device__ static __forceinline__ void metric(const MetricDesc&, const double*, const double* v, double* g, double* gi) {
+    double gv[2];
+    entry(v, 0, 0, gv);
+    g[0] = -1.0; g[5] = 1.0; g[10] = gv[0]; g[15] = gv[1];
+    morris_thorne_inverse(gv, gi);
+  }
+};
+
+template <>
+struct PointMetric<KIND_SCHWARZSCHILD> {
+  using ST = Stencil<KIND_SCHWARZSCHILD>;
+  static constexpr int NG = 8, ND = SCHWARZSCHILD_DIFFS, GMASK = 0x8421;
+  static constexpr int NV = 0;
+  __device__ static __forceinline__ void values(const MetricDesc&, const double*, double*, double*) {}
+  // christoffel_schw's entries: t_tr, r_tt, r_rr, r_thth, r_phph, 1/r, th_phph, cot
+  __device__ static __forceinline__ bool symbols(const MetricDesc& M, const double* x, const double*, int slot, double* c) {
+    double r = x[1], theta = x[2];
+    const double m = M.p[0];
+    if (slot == 1 || slot == 2) r = ST::shift(r, slot - 1);
+    if (slot >= 3) theta = ST::shift(theta, slot - 3);
+    const double f = 1.0 - sf::div(2.0 * m, r);
+    double sin_t, cos_t;
+    dm::sincos_det(theta, &sin_t, &cos_t);
+    const double gtr = sf::div(m, r * r * f);
+    c[0] = gtr;
+    c[1] = sf::div(m * f, r * r);
+    c[2] = -gtr;
+    c[3] = -(r - 2.0 * m);
+    c[4] = c[3] * sin_t * sin_t;
+    c[5] = sf::rcp(r);
+    c[6] = -sin_t * cos_t;
+    c[7] = sf::below(sin_t, 1e-8) ? 0.0 : sf::div(cos_t, sin_t);
+    return true;
+  }
+  template <class D>
+  __device__ static __forceinline__ void ricci(const double* c, D d, double* ric) { schwarzschild_ricci(c, d, ric); }
+  __device__ static constexpr int diff_place(int i) { return schwarzschild_diff_place(i); }
+  __device__ static __forceinline__ void metric(const MetricDesc& M, const double* x, const double*, double* g, double* gi) {
+    const double r = x[1], m = M.p[0];
+    const double f = 1.0 - sf::div(2.0 * m, r);
+    double sin_t, cos_t;
+    dm::sincos_det(x[2], &sin_t, &cos_t);
+    const double rr = r * r, rrss = rr * sin_t * sin_t;
+    g[0] = -f; g[5] = sf::rcp(f); g[10] = rr; g[15] = rrss;
+    gi[0] = -g[5]; gi[5] = f; gi[10] = sf::rcp(rr); gi[15] = sf::rcp(rrss);
+  }
+};
+
+// The static observer's tetrad of a point (point_tetrad) with the zero terms of
+// the Gram-Schmidt sums left out: e0 = a d_t, e1 = (b, c, 0, 0), e2 and e3 along
+// their axes. Diagonal metrics have b = 0.
+struct SparseTetrad {
+  double a, b, c, e2, e3;
+  bool ok;
+};
+template <int K>
+__device__ __forceinline__ SparseTetrad sparse_tetrad(const double* g) {
+  SparseTetrad t;
+  const double a = sf::rcp(sf::root(-g[0]));
+  t.a = a;
+  t.ok = g[0] < 0.0;
+  if (K == KIND_ALCUBIERRE) {
+    const double coeff = sf::div(g[1] * a, g[0] * a * a);
+    const double v0 = 0.0 - coeff * a;
+    const double n2 = plus_zero(g[0] * v0 * v0) + g[1] * v0 + g[1] * v0 + 1.0;
+    const double nn = sf::root(n2);
+    t.ok = t.ok && n2 > 0.0;
+    t.b = sf::div(v0, nn);
+    t.c = sf::rcp(nn);
+    t.e2 = t.e3 = 1.0;
+  } else {
+    t.b = 0.0;
+    t.c = g[5] == 1.0 ? 1.0 : sf::rcp(sf::root(g[5]));
+    t.e2 = sf::rcp(sf::root(g[10]));
+    t.e3 = sf::rcp(sf::root(g[15]));
+    t.ok = t.ok && g[5] > 0.0 && g[10] > 0.0 && g[15] > 0.0;
+  }
+  return t;
+}
+
+// what: as curvature_kernel, 1 to 6.
+template <int K, bool GRID>
+__global__ void __launch_bounds__(POINT_THREADS)
+curvature_point_kernel(const MetricDesc M, int what, const double* __restrict__ xs, int64_t n,
+                       const double* __restrict__ ks, int64_t nk, int k_shared, double* __restrict__ out, int* flags,
+                       const GridDesc grid, uint64_t seed, double* __restrict__ out2, double* __restrict__ kout) {
+  using PM = PointMetric<K>;
+  using ST = typename PM::ST;
+  extern __shared__ double smem[];
+  double* v = smem + threadIdx.x;                                // [NV][THREADS]
+  double* diff = smem + PM::NV * POINT_THREADS + threadIdx.x;    // [axes][ND][THREADS]
+  const int64_t pt = (int64_t)blockIdx.x * POINT_THREADS + threadIdx.x;
+  if (pt >= n) return;  // no barrier below: every thread keeps to its own column
+  double x[4];
+  if (GRID) {
+    grid_point(grid, pt, x);
+  } else {
+    x[0] = xs[4 * pt]; x[1] = xs[4 * pt + 1]; x[2] = xs[4 * pt + 2]; x[3] = xs[4 * pt + 3];
+  }
+  PM::values(M, x, v, diff);
+  const double inv_2h = 1.0 / (2.0 * FD_H);
+  double c[PM::NG];
+  unsigned big = 0;
+  bool regular = true;
+  // slots from the last to the point itself, whose symbols stay in c; the minus
+  // slot of an axis comes first and leaves its symbols in the store
+#pragma unroll 1
+  for (int sl = ST::slots - 1; sl >= 0; --sl) {
+    regular &= PM::symbols(M, x, v, sl, c);
+#pragma unroll
+    for (int i = 0; i < PM::NG; ++i) {
+      const unsigned h = 2u * sf::hi_of(c[i]);
+      big = h > big ? h : big;
+    }
+    if (sl > 0) {
+      double* row = diff + ((sl - 1) >> 1) * PM::ND * POINT_THREADS;
+      const bool minus = ((sl - 1) & 1) != 0;
+#pragma unroll
+      for (int i = 0; i < PM::NG; ++i) {
+        const int w = PM::diff_place(i);
+        if (w >= 0) row[w * POINT_THREADS] = minus ? c[i] : (c[i] - row[w * POINT_THREADS]) * inv_2h;
+      }
+    }
+  }
+  double ric[16];
+  const bool plain = regular && big < 2u * 0x7ff00000u;
+  if (plain) {
+    PM::ricci(c, [&](int axis, int i) { return diff[(axis * PM::ND + PM::diff_place(i)) * POINT_THREADS]; }, ric);
+  } else {
+    dense_ricci<K>(M, x, ric, flags);
+  }
+  if (what == 1) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) out[16 * pt + q] = ric[q];
+    return;
+  }
+  double g[16] = {}, gi[16] = {};
+  PM::metric(M, x, v, g, gi);
+  if (!plain) {  // the dense inverse and its sums
+    metric_g<K>(M, x, g);
+    if (!metric_g_inv_given<K>(M, x, g, gi)) atomicOr(flags, 1);
+  }
+  double rs = 0.0;  // curvature.rs:87-97; g^-1 is zero where g is
+#pragma unroll
+  for (int q = 0; q < 16; ++q)
+    if ((PM::GMASK >> q) & 1) rs += gi[q] * ric[q];
+  if (!plain) {
+    rs = 0.0;
+    for (int q = 0; q < 16; ++q) rs += gi[q] * ric[q];
+  }
+  if (what == 2) {
+    out[pt] = rs;
+    return;
+  }
+  const double factor = 1.0 / (8.0 * 3.141592653589793);
+  double ein[16];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {  // curvature.rs:99-110
+    ein[q] = ric[q];
+    if ((PM::GMASK >> q) & 1) ein[q] = ric[q] - sf::half(g[q]) * rs;
+    else if (!sf::finite(rs)) ein[q] = ric[q] - 0.0 * rs;
+  }
+  if (what == 3 || what == 4 || (what == 6 && out)) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) out[16 * pt + q] = what == 4 ? ein[q] * factor : ein[q];
+    if (what <= 4) return;
+  }
+  double t[16];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) t[q] = ein[q] * factor;  // curvature.rs:112-122
+  SparseTetrad tet = {};
+  if (what == 6) tet = sparse_tetrad<K>(g);
+  // T(k, k) (curvature.rs:127-136) of the point's vectors, one after another
+#pragma unroll 1
+  for (int64_t q = 0; q < nk; ++q) {
+    double k[4];
+    if (what == 6) {  // point_null_vector
+      const uint64_t h = splitmix64(seed ^ (uint64_t)(pt * nk + q));
+      const double u1 = sf::unit53(h >> 11), u2 = sf::unit53(splitmix64(h) >> 11);
+      const double z = fma(2.0, u1, -1.0);  // 2 u1 is exact
+      const double rho = sf::root(1.0 - z * z);  // not negative: |z| <= 1
+      double sp, cp;
+      dm::sincos_det(6.283185307179586 * u2, &sp, &cp);
+      const double n1 = rho * cp, n2 = rho * sp;
+      k[0] = K == KIND_ALCUBIERRE ? tet.a + n1 * tet.b : tet.a;
+      k[1] = n1 * tet.c;
+      k[2] = n2 * tet.e2;
+      k[3] = z * tet.e3;
+      if (!tet.ok) k[0] = k[1] = k[2] = k[3] = __longlong_as_double(0x7ff8000000000000LL);
+      if (kout) {
+#pragma unroll
+        for (int mu = 0; mu < 4; ++mu) kout[4 * (pt * nk + q) + mu] = k[mu];
+      }
+    } else {
+      const double* kp = k_shared ? ks + 4 * q : ks + 4 * (pt * nk + q);
+      k[0] = kp[0]; k[1] = kp[1]; k[2] = kp[2]; k[3] = kp[3];
+    }
+    double sacc = 0.0;
+#pragma unroll
+    for (int mu = 0; mu < 4; ++mu)
+#pragma unroll
+      for (int nu = 0; nu < 4; ++nu) sacc += t[4 * mu + nu] * k[mu] * k[nu];
+    (what == 6 ? out2 : out)[pt * nk + q] = sacc;
+  }
+}
+
+template <int K>
+constexpr bool has_point_kernel() {
+  return K == KIND_ALCUBIERRE || K == KIND_MORRIS_THORNE || K == KIND_SCHWARZSCHILD;
+}
+
+// The point kernel from this many points on. Below, the SMs are not full with
+// one thread per point and the time is one thread's chain of operations (254 us
+// for an Alcubierre grid point with 16 vectors, 91 and 87 us for Morris-Thorne
+// and Schwarzschild, whatever the number of points up to ~16384), while the
+// cooperative kernel's grows with the points: it takes 99 / 202 us for 3840 /
+// 8192 Alcubierre points, 59 / 81 us for 2048 / 4096 Morris-Thorne points.
+template <int K>
+constexpr int64_t point_min() {
+  return K == KIND_ALCUBIERRE ? 9216 : 5120;
+}
+
+template <int K, bool GRID>
+static cudaError_t launch_point_k(const MetricDesc& M, int what, const double* x, int64_t n, const double* k,
+                                  int64_t nk, int k_shared, double* out, int* flags, const GridDesc& grid,
+                                  uint64_t seed, double* out2, double* kout, cudaStream_t s) {
+  using PM = PointMetric<K>;
+  constexpr int axes = PM::ST::k;
+  const size_t smem = (size_t)(PM::NV + axes * PM::ND) * POINT_THREADS * sizeof(double);
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaFuncSetAttribute(curvature_point_kernel<K, GRID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    attr_set = true;
+  }
+  const int64_t blocks = (n + POINT_THREADS - 1) / POINT_THREADS;
+  curvature_point_kernel<K, GRID><<<(unsigned)blocks, POINT_THREADS, smem, s>>>(M, what, x, n, k, nk, k_shared, out,
+                                                                                flags, grid, seed, out2, kout);
+  return cudaGetLastError();
+}
+
 template <int K, bool GRID>
 static cudaError_t launch_curv_k(const MetricDesc& M, int what, const double* x, int64_t n, const double* k,
                                  int64_t nk, int k_shared, double* out, int* flags, const GridDesc& grid,
                                  uint64_t seed, double* out2, double* kout, cudaStream_t s) {
+  if constexpr (has_point_kernel<K>()) {
+    if (what != 0 && n >= point_min<K>())
+      return launch_point_k<K, GRID>(M, what, x, n, k, nk, k_shared, out, flags, grid, seed, out2, kout, s);
+  }
   const size_t smem = curv_smem_doubles<K>() * sizeof(double);
   static bool attr_set = false;
   if (!attr_set) {

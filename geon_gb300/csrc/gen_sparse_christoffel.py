@@ -1,7 +1,8 @@
 """Generate sparse FP64 Christoffel symbols that are bit-identical to the dense
 finite-difference fallback of the reference (metric/mod.rs:25-69 with
 types.rs:34-47's inverse), for the metrics that use it (Alcubierre,
-Morris-Thorne). Output: christoffel_sparse.cuh in this directory.
+Morris-Thorne), and the sparse curvature of one point. Output:
+christoffel_sparse.cuh and curvature_sparse.cuh in this directory.
 
 Method: run the dense algorithm symbolically. A value is an exact constant
 (0, +-1), or a runtime expression. Only operations between runtime values, or
@@ -175,6 +176,156 @@ def rhs_terms(gen, G):
                 sacc = gen.acc(sacc, t)
         lines.append(f"  k[{4 + mu}] = -({sacc.c()});" if not sacc.is_zero() else f"  k[{4 + mu}] = -0.0;")
     return lines
+
+
+# ---------------------------------------------------------------------------
+# Compact Christoffel symbols and curvature of one point (one thread per point
+# in curvature_fp64.cu): only the entries that are not structurally zero, each
+# distinct value once, and the Ricci tensor from them and their differences with
+# every structurally zero term of curvature.rs:48-85 dropped.
+# ---------------------------------------------------------------------------
+class Shared(Gen):
+    """A generator in which equal expressions are one value, so that x - x of
+    one value is an exact zero (for finite values; the kernel sends a point with
+    a non-finite symbol to the dense code), and 0.5 x halves the exponent."""
+
+    def __init__(self):
+        super().__init__()
+        self.seen = {}
+
+    def tmp(self, expr):
+        if expr.startswith("0.5 * "):
+            expr = f"sf::half({expr[6:]})"
+        if expr not in self.seen:
+            self.seen[expr] = super().tmp(expr)
+        return self.seen[expr]
+
+    def sub(self, a, b):
+        if a.expr is not None and a.expr == b.expr:
+            return ZERO
+        return super().sub(a, b)
+
+
+def used_lines(lines, results):
+    """The assignments that the results depend on, in order."""
+    need = {v.expr for v in results if v.expr}
+    keep = []
+    for line in reversed(lines):
+        m = re.match(r"\s*const double (t\d+) = (.*);$", line)
+        if m and m.group(1) not in need:
+            continue
+        keep.append(line)
+        need.update(re.findall(r"\bt\d+\b", m.group(2) if m else line))
+    return keep[::-1]
+
+
+def distinct(G):
+    """(values, index of each of the 64 entries in them or -1)."""
+    values, index = [], []
+    for v in G:
+        if v.is_zero():
+            index.append(-1)
+            continue
+        key = v.c()
+        if key not in values:
+            values.append(key)
+        index.append(values.index(key))
+    return values, index
+
+
+def ricci(gen, index, depends_on):
+    """curvature.rs:48-85 over the compact symbols: c[i] at the point, d_a[i] the
+    central difference along axis a (curvature.rs:25-46; zero off depends_on)."""
+    def g(mu, al, be):
+        i = index[16 * mu + 4 * al + be]
+        return ZERO if i < 0 else V(expr=f"c[{i}]")
+
+    def dg(axis, mu, al, be):
+        i = index[16 * mu + 4 * al + be]
+        return ZERO if i < 0 or axis not in depends_on else V(expr=f"d({depends_on.index(axis)}, {i})")
+
+    out = []
+    for mu in range(4):
+        for nu in range(4):
+            total = ZERO
+            for al in range(4):
+                term1, term2 = dg(al, al, nu, mu), dg(nu, al, al, mu)
+                term3, term4 = ZERO, ZERO
+                for la in range(4):
+                    term3 = gen.acc(term3, gen.mul(g(al, al, la), g(la, nu, mu)))
+                    term4 = gen.acc(term4, gen.mul(g(al, nu, la), g(la, al, mu)))
+                total = gen.acc(total, gen.sub(gen.add(gen.sub(term1, term2), term3), term4))
+            out.append(total)
+    return out
+
+
+def build_compact(name, spec, depends_on):
+    """The compact symbols and the inverse metric from metric values (gv as in
+    christoffel_{name}_from), and the Ricci tensor from the symbols."""
+    gen = Shared()
+    names = []
+    for row in spec:
+        for v in row:
+            if v not in ("zero", "one", "mone") and v not in names:
+                names.append(v)
+    tags = ["_c"] + [f"_{pm}{a}" for a in depends_on for pm in ("p", "m")]
+    unpack = [f"  const double {nm}{tag} = gv[{ti * len(names) + ni}];"
+              for ti, tag in enumerate(tags) for ni, nm in enumerate(names)]
+    g0 = metric_matrix(gen, spec, "_c")
+    dgv = [[[ZERO] * 4 for _ in range(4)] for _ in range(4)]
+    for al in depends_on:
+        gp, gm = metric_matrix(gen, spec, f"_p{al}"), metric_matrix(gen, spec, f"_m{al}")
+        for mu in range(4):
+            for nu in range(4):
+                d = gen.sub(gp[mu][nu], gm[mu][nu])
+                dgv[al][mu][nu] = ZERO if d.const is not None else gen.div(d, V(expr="two_h"))
+    G = christoffel(gen, g0, dgv)
+    values, index = distinct(G)
+    results = [V(expr=v) for v in values]
+    out = [f"// {name}: the {len(values)} distinct nonzero symbols from the metric values",
+           f"constexpr int {name.upper()}_GAMMAS = {len(values)};",
+           f"__device__ __forceinline__ bool {name}_gammas(const double* gv, double* c) {{", "  bool singular;"]
+    out += unpack + ["  const double two_h = 2.0 * FD_H;"] + used_lines(gen.lines, results)
+    out += [f"  c[{i}] = {v};" for i, v in enumerate(values)]
+    out += ["  return !singular;", "}"]
+    inv = Shared()
+    gi, _ = inv4(inv, metric_matrix(inv, spec, "_c"))
+    out += ["", f"// {name}: g^-1 (types.rs:34-47) of the point's metric values, zero entries not written",
+            f"__device__ __forceinline__ void {name}_inverse(const double* gv, double* gi) {{"]
+    out += [f"  const double {nm}_c = gv[{ni}];" for ni, nm in enumerate(names)] + used_lines(inv.lines, gi)
+    out += [f"  gi[{q}] = {v.c()};" for q, v in enumerate(gi) if not v.is_zero()] + ["}"]
+    return "\n".join(out) + "\n\n" + ricci_text(name, index, depends_on)
+
+
+def ricci_text(name, index, depends_on):
+    gen = Shared()
+    ric = ricci(gen, index, depends_on)
+    out = [f"// {name}: Ricci (curvature.rs:72-85) from the symbols c and their differences d(axis, i)",
+           "template <class D>",
+           f"__device__ __forceinline__ void {name}_ricci(const double* c, D d, double* ric) {{"]
+    body = used_lines(gen.lines, ric) + [f"  ric[{q}] = {v.c()};" for q, v in enumerate(ric)] + ["}"]
+    # the symbols whose differences are read, and their places in the kernel's store
+    n = max(index) + 1
+    used = sorted({int(i) for i in re.findall(r"d\(\d+, (\d+)\)", "\n".join(body))})
+    place = [used.index(i) if i in used else -1 for i in range(n)]
+    head = [f"// {name}: the {len(used)} symbols whose differences the Ricci tensor reads (place, or -1)",
+            f"constexpr int {name.upper()}_DIFFS = {len(used)};",
+            f"__device__ constexpr int {name}_diff_place(int i) {{",
+            f"  constexpr int place[{n}] = {{{', '.join(str(v) for v in place)}}};", "  return place[i];", "}"]
+    return "\n".join(head + out + body)
+
+
+# Schwarzschild's analytic symbols (schwarzschild.rs:61-107) in the order of
+# schwarzschild_gammas in curvature_fp64.cu.
+SCHW_GAMMAS = {(0, 0, 1): 0, (0, 1, 0): 0, (1, 0, 0): 1, (1, 1, 1): 2, (1, 2, 2): 3, (1, 3, 3): 4, (2, 1, 2): 5, (2, 2, 1): 5,
+               (2, 3, 3): 6, (3, 1, 3): 5, (3, 3, 1): 5, (3, 2, 3): 7, (3, 3, 2): 7}
+
+
+def schwarzschild_index():
+    index = [-1] * 64
+    for (mu, al, be), i in SCHW_GAMMAS.items():
+        index[16 * mu + 4 * al + be] = i
+    return index
 
 
 def metric_matrix(gen, spec, tag):
@@ -351,9 +502,26 @@ def header_text():
     return header + "\n" + alc + "\n\n" + mt + "\n"
 
 
+def curvature_text():
+    """The text of curvature_sparse.cuh."""
+    header = """// GENERATED by gen_sparse_christoffel.py - do not edit by hand.
+//
+// Curvature of one point with the structurally zero terms left out: the
+// distinct nonzero Christoffel symbols, the inverse metric and the Ricci tensor,
+// in the dense algorithm's order (curvature.rs:48-85), so finite results have
+// the dense code's bits up to the sign of a zero.
+#pragma once
+"""
+    return "\n\n".join([header.rstrip() + "\n", build_compact("alcubierre", ALC_SPEC, ALC_DEPENDS),
+                        build_compact("morris_thorne", MT_SPEC, MT_DEPENDS),
+                        ricci_text("schwarzschild", schwarzschild_index(), (1, 2))]) + "\n"
+
+
 def main():
     with open(os.path.join(HERE, "christoffel_sparse.cuh"), "w") as f:
         f.write(header_text())
+    with open(os.path.join(HERE, "curvature_sparse.cuh"), "w") as f:
+        f.write(curvature_text())
     for name, c in op_counts().items():
         print(f"{name}: {c['ops_per_rhs']} per right-hand side, {c['flops_per_step']} flops per RK4 step")
 

@@ -78,6 +78,26 @@ GEON_SF bool finite(double x) { return (hi_of(x) & 0x7ff00000u) != 0x7ff00000u; 
 // |x| < t for a positive t (false for NaN): magnitudes order like their bits
 GEON_SF bool below(double x, double t) { return (bits(x) & 0x7fffffffffffffffull) < bits(t); }
 
+// 0.5 * x by its exponent
+GEON_SF double half(double x) {
+  const uint32_t h = hi_of(x), l = lo_of(x), e = h & 0x7ff00000u;
+  if (e - 0x00200000u < 0x7fd00000u) return from_words(h - 0x00100000u, l);  // normal, and so is the half
+  if (((h << 1) | l) == 0u) return x;
+  return 0.5 * x;
+}
+
+// (double)v * 2^-53 for v < 2^53 (exact)
+GEON_SF double unit53(uint64_t v) {
+  if (v == 0) return 0.0;
+#ifdef __CUDA_ARCH__
+  const int z = __clzll((long long)v);
+#else
+  const int z = __builtin_clzll(v);
+#endif
+  const uint64_t m = v << (z - 11);  // leading bit at 2^52
+  return from_words((uint32_t)(m >> 32) + ((uint32_t)(1032 - z) << 20), (uint32_t)m);
+}
+
 // Estimates of 1/x (x in [1, 2]) and 1/sqrt(x) (x in [1, 4]) as FP32 bits,
 // relative error at most 2^-23 and 2^-22.4 (PTX rcp.approx, rsqrt.approx). On
 // the host `est_error` moves them by units in the last place (tests).
