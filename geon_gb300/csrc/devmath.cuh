@@ -82,13 +82,14 @@ constexpr double EX_Q5 = -0x1.afdb76e09c32dp-23;
 // only the two high words that hold a crossing need the product itself. That
 // keeps a multiplication, a rounding and a conversion (51 cycles of the FP64
 // pipe per warp) out of the common case.
-__device__ __forceinline__ void quadrant(double x, double& k, int& q) {
+__device__ __forceinline__ bool quadrant_by_word(double x, double& k, int& q) {
   const unsigned hx = sf::hi_of(x);
-  if (hx < 0x400f6a7au && hx != 0x3fe921fbu && hx != 0x4002d97cu) {  // 0 <= x < 5 pi/4
-    q = (hx > 0x3fe921fbu ? 1 : 0) + (hx > 0x4002d97cu ? 1 : 0);
-    k = sf::from_words(q == 0 ? 0u : (q == 1 ? 0x3ff00000u : 0x40000000u), 0u);
-    return;
-  }
+  q = (hx > 0x3fe921fbu ? 1 : 0) + (hx > 0x4002d97cu ? 1 : 0);
+  k = sf::from_words(q == 0 ? 0u : (q == 1 ? 0x3ff00000u : 0x40000000u), 0u);
+  return hx < 0x400f6a7au && hx != 0x3fe921fbu && hx != 0x4002d97cu;  // 0 <= x < 5 pi/4
+}
+__device__ __forceinline__ void quadrant(double x, double& k, int& q) {
+  if (quadrant_by_word(x, k, q)) return;
   k = rint(x * TWO_OVER_PI);
   // Below 2^52 the integer conversion is exact and two's-complement & 3 is the
   // mathematical residue; above it k is an even integer and the double formula
@@ -100,21 +101,17 @@ __device__ __forceinline__ void quadrant(double x, double& k, int& q) {
   }
 }
 
-__device__ __forceinline__ void sincos_det(double x, double* sp, double* cp) {
-  if (!sf::finite(x)) {
-    const double nan = __longlong_as_double(0x7ff8000000000000LL);
-    *sp = nan;
-    *cp = nan;
-    return;
-  }
-  double k;
-  int q;
-  quadrant(x, k, q);
-  const double r1 = fma(-k, PIO2_1, x);
-  const double t = fma(-k, PIO2_2, r1);
-  const double d = r1 - t;
-  const double tl = fma(-k, PIO2_3, fma(-k, PIO2_2, d));
-  const double z = t * t;
+// Multiplication by the FP64 pipe, or in the integer pipes (sf::mul: the same
+// bits for operands that sf::spread admits).
+template <bool SOFT>
+__device__ __forceinline__ double mul(double a, double b) {
+  return SOFT ? sf::mul(a, b) : a * b;
+}
+
+// sin and cos of the reduced argument t + tl in quadrant q.
+template <bool SOFT>
+__device__ __forceinline__ void sincos_reduced(double t, double tl, int q, double* sp, double* cp) {
+  const double z = mul<SOFT>(t, t);
   double ps = S17;
   ps = fma(ps, z, S15);
   ps = fma(ps, z, S13);
@@ -123,7 +120,7 @@ __device__ __forceinline__ void sincos_det(double x, double* sp, double* cp) {
   ps = fma(ps, z, S7);
   ps = fma(ps, z, S5);
   ps = fma(ps, z, S3);
-  const double tz = t * z;
+  const double tz = mul<SOFT>(t, z);
   const double wc = fma(-0.5, z, 1.0);  // 1 - z / 2 (the product is exact)
   const double sv = t + fma(tz, ps, tl * wc);
   double pc = C18;
@@ -135,7 +132,7 @@ __device__ __forceinline__ void sincos_det(double x, double* sp, double* cp) {
   pc = fma(pc, z, C6);
   pc = fma(pc, z, C4);
   const double zl = fma(t, t, -z);
-  const double cv = wc + (fma(-0.5, z, 1.0 - wc) + (fma(z * z, pc, -0.5 * zl) - tl * t));
+  const double cv = wc + (fma(-0.5, z, 1.0 - wc) + (fma(mul<SOFT>(z, z), pc, SOFT ? -sf::half_inside(zl) : -0.5 * zl) - tl * t));
   double s, c;
   if (q == 0) { s = sv; c = cv; }
   else if (q == 1) { s = cv; c = -sv; }
@@ -143,6 +140,34 @@ __device__ __forceinline__ void sincos_det(double x, double* sp, double* cp) {
   else { s = -cv; c = sv; }
   *sp = s;
   *cp = c;
+}
+
+// The reduced argument of a finite x: x - k pi/2 = t + tl. BY_WORD: only where
+// the high word tells the quadrant (else false, and the results mean nothing).
+template <bool BY_WORD>
+__device__ __forceinline__ bool reduce(double x, double* t, double* tl, int* q) {
+  double k;
+  bool ok = true;
+  if (BY_WORD) ok = quadrant_by_word(x, k, *q);
+  else quadrant(x, k, *q);
+  const double r1 = fma(-k, PIO2_1, x);
+  *t = fma(-k, PIO2_2, r1);
+  const double d = r1 - *t;
+  *tl = fma(-k, PIO2_3, fma(-k, PIO2_2, d));
+  return ok;
+}
+
+__device__ __forceinline__ void sincos_det(double x, double* sp, double* cp) {
+  if (!sf::finite(x)) {
+    const double nan = __longlong_as_double(0x7ff8000000000000LL);
+    *sp = nan;
+    *cp = nan;
+    return;
+  }
+  double t, tl;
+  int q;
+  reduce<false>(x, &t, &tl, &q);
+  sincos_reduced<false>(t, tl, q, sp, cp);
 }
 
 __device__ __forceinline__ unsigned hi_word(double x) {

@@ -470,6 +470,59 @@ __device__ __forceinline__ void metric_asymptotic_direction(const MetricDesc& M,
 }
 
 
+// Schwarzschild momentum derivatives k[4..7] at y, sin and cos of theta given:
+// schwarzschild.rs:61-107 fused with the sum of geodesic.rs:49-57; only the
+// nonzero entries contribute (alpha-major, beta-minor order kept). SOFT: the
+// multiplications in the integer pipes; returns the largest sf::spread of their
+// operands (the result stands if it is below sf::RANGE).
+template <bool SOFT>
+__device__ __forceinline__ uint32_t schw_rhs_at(double m, const double y[8], double sin_t, double cos_t, double k[8]) {
+  const double p0 = y[4], p1 = y[5], p2 = y[6], p3 = y[7];
+  const double r = y[1];
+  auto mul = [](double a, double b) { return dm::mul<SOFT>(a, b); };
+  auto div = [](double a, double b) { return SOFT ? sf::div_inside(a, b) : sf::div(a, b); };
+  const double f = 1.0 - div(2.0 * m, r);
+  const double rr = mul(r, r);
+  const double rrf = mul(rr, f);
+  const double gtr = div(m, rrf);   // Gamma^t_tr = Gamma^t_rt = -Gamma^r_rr
+  const double g_r_tt = div(mul(m, f), rr);  // Gamma^r_tt
+  const double r2m = r - 2.0 * m;              // -Gamma^r_thth
+  const double ir = SOFT ? sf::rcp_inside(r) : sf::rcp(r);                // Gamma^th_rth, Gamma^ph_rph
+  const bool pole = sf::below(sin_t, 1e-8);
+  const double cot = !SOFT && pole ? 0.0 : div(cos_t, sin_t);
+  // Products shared between the sums; a negated entry is a subtracted term
+  // (x + (-y) is x - y, and (-a) b c is -((a b) c), bit for bit).
+  const double gp1 = mul(gtr, p1), irp1 = mul(ir, p1);
+  double s;
+  s = plus_zero(mul(mul(gtr, p0), p1));
+  s += mul(gp1, p0);
+  k[4] = -s;
+  s = plus_zero(mul(mul(g_r_tt, p0), p0));
+  s -= mul(gp1, p1);
+  s -= mul(mul(r2m, p2), p2);
+  s -= mul(mul(mul(mul(r2m, sin_t), sin_t), p3), p3);
+  k[5] = -s;
+  s = plus_zero(mul(irp1, p2));
+  s += mul(mul(ir, p2), p1);
+  s -= mul(mul(mul(sin_t, cos_t), p3), p3);
+  k[6] = -s;
+  s = plus_zero(mul(irp1, p3));
+  s += mul(mul(cot, p2), p3);
+  s += mul(mul(ir, p3), p1);
+  s += mul(mul(cot, p3), p2);
+  k[7] = -s;
+  uint32_t worst = SOFT && pole ? sf::RANGE : 0;
+  if (SOFT) {
+    const double all[15] = {p0, p1, p2, p3, r, f, m, gtr, g_r_tt, r2m, cot, sin_t, cos_t, rr, rrf};
+#pragma unroll
+    for (int i = 0; i < 15; ++i) {
+      const uint32_t d = sf::spread(all[i]);
+      worst = d > worst ? d : worst;
+    }
+  }
+  return worst;
+}
+
 // ---------------------------------------------------------------------------
 // Geodesic right-hand side (geodesic.rs:38-59): k = (p, -Gamma^mu_ab p^a p^b).
 // ---------------------------------------------------------------------------
@@ -482,39 +535,9 @@ __device__ __forceinline__ bool geodesic_rhs(const MetricDesc& M, const double y
     k[4] = -0.0; k[5] = -0.0; k[6] = -0.0; k[7] = -0.0;
     return true;
   } else if (K == KIND_SCHWARZSCHILD) {
-    // schwarzschild.rs:61-107 fused with the sum; only the nonzero entries
-    // contribute (alpha-major, beta-minor order kept).
-    const double r = y[1], theta = y[2], m = M.p[0];
-    const double f = 1.0 - sf::div(2.0 * m, r);
     double sin_t, cos_t;
-    dm::sincos_det(theta, &sin_t, &cos_t);
-    const double rr = r * r;
-    const double gtr = sf::div(m, rr * f);      // Gamma^t_tr = Gamma^t_rt = -Gamma^r_rr
-    const double g_r_tt = sf::div(m * f, rr);   // Gamma^r_tt
-    const double r2m = r - 2.0 * m;             // -Gamma^r_thth
-    const double ir = sf::rcp(r);               // Gamma^th_rth, Gamma^ph_rph
-    const double cot = sf::below(sin_t, 1e-8) ? 0.0 : sf::div(cos_t, sin_t);
-    // Products shared between the sums; a negated entry is a subtracted term
-    // (x + (-y) is x - y, and (-a) b c is -((a b) c), bit for bit).
-    const double gp1 = gtr * p1, irp1 = ir * p1;
-    double s;
-    s = plus_zero(gtr * p0 * p1);
-    s += gp1 * p0;
-    k[4] = -s;
-    s = plus_zero(g_r_tt * p0 * p0);
-    s -= gp1 * p1;
-    s -= r2m * p2 * p2;
-    s -= r2m * sin_t * sin_t * p3 * p3;
-    k[5] = -s;
-    s = plus_zero(irp1 * p2);
-    s += ir * p2 * p1;
-    s -= sin_t * cos_t * p3 * p3;
-    k[6] = -s;
-    s = plus_zero(irp1 * p3);
-    s += cot * p2 * p3;
-    s += ir * p3 * p1;
-    s += cot * p3 * p2;
-    k[7] = -s;
+    dm::sincos_det(y[2], &sin_t, &cos_t);
+    schw_rhs_at<false>(M.p[0], y, sin_t, cos_t, k);
     return true;
   } else if (K == KIND_ALCUBIERRE) {
     return rhs_alcubierre_sparse(M, y, k);
@@ -580,6 +603,59 @@ __device__ __forceinline__ bool rk4_step(const MetricDesc& M, const double y[8],
   }
   *finite = fin;
   return ok;
+}
+
+// rk4_step of Schwarzschild with its multiplications in the integer pipes:
+// about 220 of the step's 390 FP64 operations stay on the FP64 pipe, which both
+// kinds of pipe then share evenly. The same bits; false (out not written) when an
+// operand is outside the range of sf::mul (a zero momentum, a pole, the horizon)
+// and the step is rk4_step's.
+__device__ __forceinline__ bool rk4_step_schw_soft(const MetricDesc& M, const double y[8], double h, double half_h,
+                                                   double sixth, double out[8], bool* finite) {
+  double k[8], acc[8], ys[8];
+  uint32_t worst = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) ys[i] = y[i];
+  const double m = M.p[0];
+#pragma unroll 1
+  for (int stage = 0;; ++stage) {
+    double t, tl, sin_t, cos_t;
+    int q;
+    if (!dm::reduce<true>(ys[2], &t, &tl, &q)) worst = sf::RANGE;
+    dm::sincos_reduced<true>(t, tl, q, &sin_t, &cos_t);
+    uint32_t d = sf::spread(t);
+    worst = d > worst ? d : worst;
+    d = schw_rhs_at<true>(m, ys, sin_t, cos_t, k);
+    worst = d > worst ? d : worst;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) k[i] = ys[4 + i];
+#pragma unroll
+    for (int i = 4; i < 8; ++i) {
+      d = sf::spread(k[i]);
+      worst = d > worst ? d : worst;
+    }
+    if (stage == 3) break;
+    const double c = stage < 2 ? half_h : h;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      acc[i] = stage == 0 ? k[i] : fma(2.0, k[i], acc[i]);
+      ys[i] = y[i] + sf::mul(c, k[i]);
+    }
+  }
+  bool fin = true;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const double sum = acc[i] + k[i];
+    const uint32_t d = sf::spread(sum);
+    worst = d > worst ? d : worst;
+    out[i] = y[i] + sf::mul(sixth, sum);
+    fin &= sf::finite(out[i]);
+  }
+  const uint32_t ds = sf::spread(sixth), dh = sf::spread(half_h);
+  worst = ds > worst ? ds : worst;
+  worst = dh > worst ? dh : worst;
+  *finite = fin;
+  return worst < sf::RANGE - (2u << 21);  // h itself is twice half_h
 }
 
 // Residual |g(p, p)| at the position of y (geodesic.rs:82-84), dense dot4.

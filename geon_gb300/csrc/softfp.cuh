@@ -86,6 +86,15 @@ GEON_SF double half(double x) {
   return 0.5 * x;
 }
 
+// 0.5 * x for x zero or in [2^-1000, inf): no branch
+GEON_SF double half_inside(double x) {
+  const uint32_t h = hi_of(x), l = lo_of(x);
+  return from_words(((h << 1) | l) ? h - 0x00100000u : h, l);
+}
+
+// -2 * x for a normal x whose double is finite: no branch
+GEON_SF double minus_twice_inside(double x) { return from_words((hi_of(x) ^ 0x80000000u) + 0x00100000u, lo_of(x)); }
+
 // (double)v * 2^-53 for v < 2^53 (exact)
 GEON_SF double unit53(uint64_t v) {
   if (v == 0) return 0.0;
@@ -186,13 +195,9 @@ GEON_SF uint32_t reciprocal_estimate(uint64_t B) {
   return fixed31(rcp_bits(f));
 }
 
-// a / b, rounded to nearest: the bits of the IEEE division.
-GEON_SF double div(double a, double b) {
+// a / b for operands in [2^-255, 2^257)
+GEON_SF double div_inside(double a, double b) {
   const uint32_t ah = hi_of(a), al = lo_of(a), bh = hi_of(b), bl = lo_of(b);
-  if (outside(bh) | outside(ah)) {
-    if ((((ah << 1) | al) | outside(bh)) == 0u) return from_words((ah ^ bh) & 0x80000000u, 0u);  // +-0 / b
-    return a / b;
-  }
   const uint32_t am = (ah & 0xfffffu) | 0x100000u, bm = (bh & 0xfffffu) | 0x100000u;
   const uint64_t B = pack(bm, bl);
   uint64_t A = pack(am, al);
@@ -204,10 +209,19 @@ GEON_SF double div(double a, double b) {
   return from_words(h, (uint32_t)Q);
 }
 
-// 1 / b
-GEON_SF double rcp(double b) {
+// a / b, rounded to nearest: the bits of the IEEE division.
+GEON_SF double div(double a, double b) {
+  const uint32_t ah = hi_of(a), bh = hi_of(b);
+  if (outside(bh) | outside(ah)) {
+    if ((((ah << 1) | lo_of(a)) | outside(bh)) == 0u) return from_words((ah ^ bh) & 0x80000000u, 0u);  // +-0 / b
+    return a / b;
+  }
+  return div_inside(a, b);
+}
+
+// 1 / b for b in [2^-255, 2^257)
+GEON_SF double rcp_inside(double b) {
   const uint32_t bh = hi_of(b), bl = lo_of(b);
-  if (outside(bh)) return 1.0 / b;
   const uint32_t bm = (bh & 0xfffffu) | 0x100000u;
   const uint64_t B = pack(bm, bl);
   const uint32_t less = (bl | (bm ^ 0x100000u)) ? 1u : 0u;  // B is not a power of two
@@ -215,6 +229,9 @@ GEON_SF double rcp(double b) {
   const uint32_t h = (uint32_t)(Q >> 32) + (1022u << 20) - (bh - bm) + (1022u << 20) - (less << 20);
   return from_words(h, (uint32_t)Q);
 }
+
+// 1 / b
+GEON_SF double rcp(double b) { return outside(hi_of(b)) ? 1.0 / b : rcp_inside(b); }
 
 // sqrt(a), rounded to nearest: the bits of the IEEE square root. With n in
 // [1, 4) the significand (times 2 for an odd exponent), A = n 2^52, and y the
@@ -249,6 +266,43 @@ GEON_SF double root(double a) {
   const uint64_t M = S + ((int64_t)(R3 - S) > 0 ? 1u : 0u);
   const uint32_t h = (uint32_t)(M >> 32) + ((((ah >> 20) - odd + 1021u) >> 1) << 20);
   return from_words(h, (uint32_t)M);
+}
+
+// How far |x| is from the middle of the range of mul's operands: below RANGE
+// exactly when |x| is in [2^-170, 2^170). A kernel takes the largest over all
+// operands it starts from and tests it once; products of up to six of them are
+// then normal numbers, whatever the order.
+constexpr uint32_t RANGE = 340u << 21;
+GEON_SF uint32_t spread(double x) { return hi_of(x) * 2u - ((1023u - 170u) << 21); }
+
+// a * b, rounded to nearest even, for normal operands whose product is normal:
+// the bits of the IEEE multiplication in 15 cycles of the integer pipes (the
+// FP64 pipe takes 19; sharing the multiplications between both brings a
+// multiplication to 9.6). The significands are multiplied exactly in 32-bit
+// pieces, a's moved up 11 bits so that the leading word of the product is the
+// result's significand or half of it; the words below it round.
+GEON_SF double mul(double a, double b) {
+  const uint32_t ah = hi_of(a), al = lo_of(a), bh = hi_of(b), bl = lo_of(b);
+  const uint32_t am = (ah & 0xfffffu) | 0x100000u, bm = (bh & 0xfffffu) | 0x100000u;
+  const uint64_t A = pack(am, al) << 11;
+  const uint32_t A1 = (uint32_t)(A >> 32), A0 = (uint32_t)A;
+  const uint64_t ll = (uint64_t)A0 * bl;
+  const uint64_t m1 = (uint64_t)A1 * bl + (uint32_t)(ll >> 32);
+  const uint64_t m2 = (uint64_t)A0 * bm + (uint32_t)m1;
+  const uint64_t hh = (uint64_t)A1 * bm + ((uint64_t)(uint32_t)(m1 >> 32) + (uint32_t)(m2 >> 32));
+  const uint32_t h1 = (uint32_t)(hh >> 32), w = (uint32_t)m2;
+  const uint32_t sh = ((h1 >> 20) & 1u) ^ 1u;  // the product's significand is below 2
+#ifdef __CUDA_ARCH__
+  const uint64_t top = pack(__funnelshift_l((uint32_t)hh, h1, sh), __funnelshift_l(w, (uint32_t)hh, sh));
+#else
+  const uint64_t top = sh ? (hh << 1) | (w >> 31) : hh;
+#endif
+  // what is below, its last bit sticky: half or more rounds up, exactly half to even
+  const uint32_t below_top = (w << sh) | ((uint32_t)ll ? 1u : 0u);
+  const uint64_t carry = (uint64_t)below_top + (0x7fffffffu + ((uint32_t)top & 1u));
+  const uint64_t m = top + (carry >> 32);
+  const uint32_t h = (uint32_t)(m >> 32) + (ah - am) + (bh - bm) - (1021u << 20) - (sh << 20);
+  return from_words(h, (uint32_t)m);
 }
 
 }  // namespace sf

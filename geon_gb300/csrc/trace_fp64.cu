@@ -64,7 +64,9 @@ struct Fp64Stepper {
   __device__ __forceinline__ int step(const TraceLaunch& L) {
     double yn[8];
     bool finite;
-    singular |= !rk4_step<K>(L.M, y, L.step, L.half_step, L.sixth, yn, &finite);
+    if (K != KIND_SCHWARZSCHILD ||
+        !rk4_step_schw_soft(L.M, y, L.step, L.half_step, L.sixth, yn, &finite))
+      singular |= !rk4_step<K>(L.M, y, L.step, L.half_step, L.sixth, yn, &finite);
     if (!finite) return STEP_NONFINITE;
 #pragma unroll
     for (int i = 0; i < 8; ++i) y[i] = yn[i];
@@ -175,7 +177,7 @@ cudaError_t launch_trace_multi_fp64(const TraceLaunch* jobs, const MultiDesc& D,
 // Alcubierre view of 5000 steps from 653 to 487 ms, bit for bit (and to 34.5 ms
 // with alcubierre_flat_steps).
 template <int K, int SRC, int SINK>
-__global__ void __launch_bounds__(FP64_BLOCK) trace_fp64_kernel(const TraceLaunch L) {
+__global__ void __launch_bounds__(FP64_BLOCK, K == KIND_SCHWARZSCHILD ? 16 : 1) trace_fp64_kernel(const TraceLaunch L) {
   trace_loop<Fp64Stepper<K>, K, SRC, SINK>(L);
 }
 

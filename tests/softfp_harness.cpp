@@ -1,5 +1,4 @@
-// Compares the integer division, reciprocal and square root of softfp.cuh with
-// the host's IEEE operations, bit for bit; prints the number of differences.
+// Compares the integer operations of softfp.cuh with the host's IEEE operations, bit for bit; prints the number of differences.
 // argv: pattern of the significands (0-7), random cases, shift of the estimates
 // in units in the last place.
 #include <stdio.h>
@@ -48,20 +47,35 @@ int main(int argc, char** argv) {
     bad += !same(sf::root(a), sqrt(a));
     bad += !same(sf::root(fabs(a)), sqrt(fabs(a)));
     // next to exact quotients and squares
-    const double p = a * b, q = fabs(a) * fabs(a);
+    const double p = a * b, q = fabs(a) * fabs(a);  // (a b may leave the normal range)
     uint64_t up = sf::bits(p) + rng() % 3 - 1, uq = sf::bits(q) + rng() % 5 - 2;
     double pp, qq;
     memcpy(&pp, &up, 8);
     memcpy(&qq, &uq, 8);
     bad += !same(sf::div(pp, b), pp / b);
     bad += !same(sf::root(qq), sqrt(qq));
+    bad += !same(sf::mul(a, b), p) && p - p == 0.0 && fabs(p) >= 0x1p-1022;
+    const double c = make(pattern, 338), d = make(i & 4 ? pattern : 0, 338), e = make(0, 338);
+    if (sf::spread(c) < sf::RANGE && sf::spread(d) < sf::RANGE && sf::spread(e) < sf::RANGE) {
+      bad += !same(sf::mul(sf::mul(c, d), e), c * d * e) + !same(sf::mul(c, c), c * c);
+      bad += !same(sf::mul(sf::mul(c, d), sf::mul(sf::mul(d, e), e)), (c * d) * ((d * e) * e));
+    } else {
+      ++bad;
+    }
+    bad += sf::half(a) != 0.5 * a;
+    bad += sf::half_inside(c) != 0.5 * c || sf::half_inside(0.0) != 0.0 || sf::minus_twice_inside(c) != -2.0 * c;
+    const uint64_t u = rng() >> 11 >> (rng() % 53);
+    bad += sf::unit53(u) != (double)u * 0x1p-53;
     bad += sf::finite(pp) != (pp - pp == 0.0);
     bad += sf::below(a, 1e-8) != (fabs(a) < 1e-8);
   }
   const double special[] = {0.0, -0.0, 1.0, -1.0, INFINITY, -INFINITY, NAN, 5e-324, 2.2250738585072014e-308, 1e-310,
-                            1.7e308, -1e308, 3.0, 0x1p-255, 0x1.fffffffffffffp-256, 0x1p257, 0x1.fffffffffffffp256,
+                            1.7e308, -1e308, 3.0, 0x1p-255, 0x1.fffffffffffffp-256, 0x1p257, 0x1.fffffffffffffp256, 0x1p-170, 0x1.fffffffffffffp-171, 0x1p170, 0x1.fffffffffffffp169,
                             1e-8, 0x1.5798ee2308c39p-27};
   for (double a : special) {
+    bad += !same(sf::half(a), 0.5 * a);
+    const double m = fabs(a);
+    bad += (sf::spread(a) < sf::RANGE) != (m >= 0x1p-170 && m < 0x1p170);
     bad += !same(sf::root(a), sqrt(a)) + !same(sf::rcp(a), 1.0 / a);
     bad += sf::finite(a) != (a - a == 0.0);
     bad += sf::below(a, 1e-8) != (fabs(a) < 1e-8);

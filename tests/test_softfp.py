@@ -1,5 +1,5 @@
-"""softfp.cuh: the integer division, reciprocal and square root of the FP64
-kernels give the bits of the IEEE operations (the host's), for every shape of
+"""softfp.cuh: the integer division, reciprocal, square root and multiplication
+of the FP64 kernels give the bits of the IEEE operations (the host's), for every shape of
 significand, next to exact quotients and squares, for special values, and with
 the hardware estimates moved to either side of their error bound."""
 import os
