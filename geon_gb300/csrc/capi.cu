@@ -36,9 +36,8 @@ std::atomic<float> g_reserve{0.0f};
 std::atomic<double> g_rtol{1e-10};  // GEON_ADAPTIVE error tolerances
 std::atomic<double> g_atol{1e-12};
 // Mixed-kernel variant per metric kind and ray source (camera/array, equatorial),
-// chosen by geon_autotune_mixed (default 0, except the equatorial source: 2, at
-// most 51 registers; the 2^20-ray sweep takes 267 ms with it, 271 without a cap).
-std::atomic<int> g_variant[4][2] = {{{0}, {0}}, {{0}, {2}}, {{0}, {0}}, {{0}, {0}}};
+// chosen by geon_autotune_mixed (default 0).
+std::atomic<int> g_variant[4][2] = {{{0}, {0}}, {{0}, {0}}, {{0}, {0}}, {{0}, {0}}};
 // Kernels launched by this library since load (ours only; memsets excluded).
 std::atomic<unsigned long long> g_launches{0};
 inline void counted(unsigned long long n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
@@ -989,15 +988,27 @@ int geon_equatorial_rays(geon_metric_t m, double r_obs, const double* alpha, siz
 
 // Classify rays launched at the given angles on stream s (device buffers).
 // Sweeps of at least SHADOW_ORDER_MIN rays (and fewer than 2^31) are claimed
-// longest first (launch_shadow_order); smaller ones in index order.
-constexpr int64_t SHADOW_ORDER_MIN = 65536;
+// longest first (launch_shadow_order); smaller ones, two warps per SM quarter and
+// less, in index order: they take as long as one ray does either way (60000 rays
+// 28.3 ms in order, 36.5 unordered; 38000 rays 20.7).
+constexpr int64_t SHADOW_ORDER_MIN = 40000;
 
 static int classify_dev(geon_metric_t m, double r_obs, const double* d_alpha, int64_t n, double step,
                         int64_t max_steps, int precision, int32_t* d_term, int64_t* d_steps,
                         cudaStream_t s) {
   DBuf ws, dorder;
-  GEON_CUDA(ws.alloc(sizeof(unsigned long long) * 4, s));
-  GEON_CUDA(cudaMemsetAsync(ws.p, 0, sizeof(unsigned long long) * 4, s));
+  // a mixed sweep that the GPU holds at once (a launch variant or reserve chosen
+  // by the caller keeps its own grid) is dealt by SM quarter: trace_resident
+  int dev = 0, sms = 0;
+  GEON_CUDA(cudaGetDevice(&dev));
+  GEON_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const bool resident = precision == GEON_MIXED && n > (int64_t)sms * 128 && n <= (int64_t)sms * 1024 &&
+                        4u * (unsigned)sms < RESIDENT_QUARTERS && g_variant[m->desc.kind][1].load() == 0 &&
+                        g_reserve.load() == 0.0f;
+  const size_t ws_bytes = sizeof(unsigned long long) * 4 +
+                          (resident ? sizeof(unsigned) * (RESIDENT_QUARTERS + (size_t)(n + 31) / 32) : 0);
+  GEON_CUDA(ws.alloc(ws_bytes, s));
+  GEON_CUDA(cudaMemsetAsync(ws.p, 0, ws_bytes, s));
   const int32_t* order = nullptr;
   if (g_sweep_order.load() && n >= SHADOW_ORDER_MIN && n < ((int64_t)1 << 31)) {
     GEON_CUDA(dorder.alloc(sizeof(int32_t) * n, s));
@@ -1015,6 +1026,11 @@ static int classify_dev(geon_metric_t m, double r_obs, const double* d_alpha, in
   L.steps = d_steps;
   L.queue = ws.as<unsigned long long>();
   L.flags = reinterpret_cast<int*>(L.queue + 1);
+  if (resident) {
+    L.started = reinterpret_cast<unsigned*>(L.queue + 4);
+    L.taken = L.started + RESIDENT_QUARTERS;
+    L.quarters = 4u * (unsigned)sms;
+  }
   GEON_CUDA(launch_trace(L, precision, SRC_EQUATORIAL, SINK_SHADOW, s));
   return GEON_OK;
 }

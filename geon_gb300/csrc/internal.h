@@ -93,6 +93,8 @@ struct MixedConsts {
   float cap_steps;                               // the step cap, for the early decision's budget test
 };
 
+constexpr unsigned RESIDENT_QUARTERS = 4096;  // more than 4 per SM of any device
+
 struct TraceLaunch {
   MetricDesc M;
   MixedConsts mx;
@@ -130,7 +132,13 @@ struct TraceLaunch {
   double rtol, atol;
   // work queue
   const int32_t* order;       // the k-th claimed ray is order[k] (null: ray k); n < 2^31 when set
-  unsigned long long* queue;  // next unclaimed ray index
+  unsigned long long* queue;  // next unclaimed ray index (zero before the launch)
+  // trace_resident (null: trace_loop): warps started per SM quarter
+  // (RESIDENT_QUARTERS counters), a flag per 32 rays, all zero before the launch;
+  // quarters: the SM quarters of the device
+  unsigned* started;
+  unsigned* taken;
+  unsigned quarters;
   int* flags;                 // bit 0: a metric became singular (inverse of g failed)
 };
 

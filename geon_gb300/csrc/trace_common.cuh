@@ -250,6 +250,67 @@ __device__ __forceinline__ void trace_loop(const TraceLaunch& L) {
 }
 
 
+// trace_loop for a sweep that the GPU holds at once (one warp per 32 rays, blocks
+// of one warp). What sets its time is the SM quarter with the most warps of long
+// rays, so pieces of 32 rays (in claim order: longest first) are dealt by
+// quarter: the l-th warp to start on quarter q takes piece l * quarters + q. With
+// warps that claimed in the order they started, 120000 rays (2152 long warps)
+// put 7 on some quarters and none on others, and blocks in index order still up
+// to 5, for 3.5 on average; dealt, every quarter has 3 or 4. A quarter with fewer
+// warps leaves pieces over: warps that are done walk all pieces once and take
+// those no one has taken (L.taken, one flag per piece).
+template <class Stepper, int K, int SRC, int SINK>
+__device__ __forceinline__ void trace_resident(const TraceLaunch& L) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned pieces = (unsigned)((L.n + 31) / 32);
+  unsigned piece = 0;
+  if (lane == 0) {
+    unsigned sm, warp;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    asm volatile("mov.u32 %0, %%warpid;" : "=r"(warp));
+    const unsigned q = (4u * sm + (warp & 3u)) % RESIDENT_QUARTERS;
+    piece = atomicAdd(&L.started[q], 1u) * L.quarters + q;
+    // another warp's flag, or no such piece: on to the walk
+    if (piece >= pieces || atomicExch(&L.taken[piece], 1u)) piece = pieces;
+  }
+  piece = __shfl_sync(FULL, piece, 0);
+  Stepper st;
+  for (;;) {
+    if (piece < pieces) {
+      const int64_t idx = 32 * (int64_t)piece + lane;
+      int64_t ray = idx < L.n ? (L.order ? (int64_t)L.order[idx] : idx) : -1;
+      int64_t n = 0;
+      if (ray >= 0) {
+        double y0[8];
+        load_ray<SRC>(L, ray, y0);
+        st.load(L, y0);
+      }
+      while (__ballot_sync(FULL, ray >= 0)) {
+        if (ray >= 0) {
+          int t = TERM_NONE;
+          int64_t taken = 0;
+          n = group_steps(st, L, L.max_steps, n, t, taken);
+          if (t != TERM_NONE) {
+            double y[8];
+            st.to_double(y);
+            store_ray<K, SINK>(L, ray, t, y, taken);
+            ray = -1;
+          }
+        }
+      }
+    }
+    if (lane == 0) {
+      do {
+        piece = (unsigned)atomicAdd(L.queue, 1ull);
+      } while (piece < pieces && atomicExch(&L.taken[piece], 1u));
+    }
+    piece = __shfl_sync(FULL, piece, 0);
+    if (piece >= pieces) break;
+  }
+  st.finish(L);
+}
+
 // ---------------------------------------------------------------------------
 // Several jobs in one persistent launch (e.g. renders of different metrics):
 // one work queue over the concatenated rays, job j owning the global indices

@@ -94,7 +94,10 @@ __device__ __forceinline__ bool ff_gt(float hi, float lo, float thi, float tlo) 
 // FEAT_DECIDE: every ray is a bisection ray whose class settles early
 // (decided_k); FEAT_DECIDE_DYN: a per-ray flag says so (the serving kernel).
 enum : int { FEAT_BAND = 1, FEAT_REPROJECT = 2, FEAT_PLANAR = 4, FEAT_PLANAR_DYN = 8, FEAT_ORBIT = 16,
-             FEAT_ORBIT_DYN = 32, FEAT_DECIDE = 64, FEAT_DECIDE_DYN = 128, FEAT_NO_TIME = 256, FEAT_OWN = 512 };
+             FEAT_ORBIT_DYN = 32, FEAT_DECIDE = 64, FEAT_DECIDE_DYN = 128, FEAT_NO_TIME = 256, FEAT_OWN = 512, FEAT_LATENCY = 1024 };
+// The step's constants in registers and its tests one by one (with FEAT_OWN): for
+// launches with a warp or less per SM quarter, where the chain of a step sets the time.
+constexpr int FEAT_CHAIN = FEAT_OWN | FEAT_LATENCY;
 
 // Right-hand side on the equatorial plane: rhs_stage at sin theta = 1,
 // cos theta = 0, p^theta = 0, where its theta terms vanish (Gamma^th_phph =
@@ -171,10 +174,9 @@ struct MixedCore {
 
   __device__ __forceinline__ void setup(const TraceLaunch& L) {
     if constexpr ((FEAT & FEAT_OWN) != 0) own = L.mx;
-    if constexpr ((FEAT & FEAT_DECIDE) != 0) {
-      // Bisection rounds keep the step's constants in registers: with one warp
-      // per SM quarter the latency of a constant-bank read shows (6.5 against
-      // 5.9 ms). Converted from the FP64 values here (the same roundings as
+    if constexpr ((FEAT & FEAT_LATENCY) != 0) {
+      // With one warp per SM quarter the latency of a constant-bank read shows
+      // (64 bisections: 6.5 against 5.9 ms), so they are in registers. Converted from the FP64 values here (the same roundings as
       // mixed_consts), because the compiler would read a plain copy again.
       own.m = __double2float_rn(L.M.p[0]);
       own.two_m = __double2float_rn(2.0 * L.M.p[0]);
@@ -640,14 +642,15 @@ struct MixedCore {
     k5 = Mt::fma(gtr, Mt::fma(-E, E, p1 * p1), rm * (p3 * p3));
     w7 = (p1 * ir) * p3;
   }
-  // Rays of kind K have fast steps. Not the bisection rounds: a ray of theirs
-  // is decided by tests between its steps, and with one warp per SM quarter a
-  // round takes as long as its slowest ray's chain of steps, which the combined
-  // test lengthens (64 brackets of 40 halvings: 7.3 ms with it, 5.9 without).
+  // Rays of kind K have fast steps. Not where one warp per SM quarter runs
+  // (FEAT_LATENCY): the time is the chain of a ray's steps, which the combined
+  // test lengthens (64 brackets of 40 halvings, whose rays are decided by tests
+  // between their steps: 7.3 ms with it, 5.9 without; a sweep of 1000 rays:
+  // 17.1 and 16.8 ms).
   template <int K>
   static constexpr bool any_fast() {
     return K == KIND_ALCUBIERRE ? (FEAT & (FEAT_BAND | FEAT_REPROJECT)) == 0
-                                : (FEAT & (FEAT_BAND | FEAT_REPROJECT | FEAT_DECIDE)) == 0 &&
+                                : (FEAT & (FEAT_BAND | FEAT_REPROJECT | FEAT_LATENCY)) == 0 &&
                                       (any_orbit<K>() || (K == KIND_SCHWARZSCHILD &&
                                                           (FEAT & (FEAT_PLANAR | FEAT_PLANAR_DYN)) != 0));
   }
@@ -828,7 +831,7 @@ struct MixedStepperAny : MixedCore<FEAT> {
 // and 9 blocks of 128 for the planar equatorial step, 59 and 8 for the camera
 // step; 8 blocks of 128: <= 64 registers; 10: <= 51), trading registers (and
 // spills) for resident warps. Measured with the combined test and the
-// constant-bank constants, before and after: the 2^20-ray sweep 274 -> 268 ms
+// constant-bank constants, before and after: the 2^20-ray sweep 274 -> 269 ms
 // (cap 10), a 960 x 540 frame with 4 samples per pixel 29.4 -> 26.9 ms. What
 // bounds the step is not its instruction count any more (144 -> 139 of them,
 // and 126 in a version that tested only every fourth step ran no faster) but
@@ -839,7 +842,8 @@ struct MixedStepperAny : MixedCore<FEAT> {
 template <int K, int SRC, int SINK, int MINB, int FEAT, int BLOCK = TRACE_BLOCK>
 __global__ void __launch_bounds__(BLOCK, MINB) trace_mixed_kernel(const TraceLaunch L) {
   constexpr int PL = (SRC == SRC_EQUATORIAL && K == KIND_SCHWARZSCHILD) ? FEAT_PLANAR : 0;
-  trace_loop<MixedStepper<K, FEAT | PL>, K, SRC, SINK>(L);
+  if constexpr (BLOCK == 32) trace_resident<MixedStepper<K, FEAT | PL>, K, SRC, SINK>(L);
+  else trace_loop<MixedStepper<K, FEAT | PL>, K, SRC, SINK>(L);
 }
 
 template <int K, int SRC, int SINK, int MINB, int FEAT, int BLOCK = TRACE_BLOCK>
@@ -861,6 +865,17 @@ static cudaError_t launch_mst_v(const TraceLaunch& L, cudaStream_t s) {
   if (grid < 1) grid = 1;
   trace_mixed_kernel<K, SRC, SINK, MINB, FEAT, BLOCK><<<grid, BLOCK, 0, s>>>(L);
   return cudaGetLastError();
+}
+
+// Rays that give every SM quarter `warps` warps.
+static int64_t rays_for(int warps) {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return (int64_t)sms * 4 * 32 * warps;
 }
 
 template <int K, int SRC, int SINK>
@@ -885,7 +900,11 @@ static cudaError_t launch_mst(const TraceLaunch& L, cudaStream_t s) {
     case FEAT_BAND | FEAT_REPROJECT: return launch_mst_v<K, SRC, SINK, 1, FEAT_BAND | FEAT_REPROJECT>(L, s);
   }
   if constexpr (SRC == SRC_EQUATORIAL && SINK == SINK_SHADOW) {
-    if (L.decide) return launch_mst_v<K, SRC, SINK, 1, FEAT_DECIDE | FEAT_OWN>(L, s);  // bisection rounds
+    if (L.decide) return launch_mst_v<K, SRC, SINK, 1, FEAT_DECIDE | FEAT_CHAIN>(L, s);  // bisection rounds
+    // one warp per SM quarter: the chain of a step sets the time (19000 rays 17.0
+    // against 17.3 ms; from two warps on the combined test is the faster one:
+    // 38000 rays 21.9 against 22.9 ms)
+    if (L.n <= rays_for(1)) return launch_mst_v<K, SRC, SINK, 1, FEAT_CHAIN>(L, s);
     // variant = register cap + 3 * block size (128, 64, 256); the same caps in
     // registers per thread (64, 51) at every block size
     switch (L.variant) {
@@ -897,13 +916,24 @@ static cudaError_t launch_mst(const TraceLaunch& L, cudaStream_t s) {
       case 6: return launch_mst_v<K, SRC, SINK, 1, 0, 256>(L, s);
       case 7: return launch_mst_v<K, SRC, SINK, 4, 0, 256>(L, s);
       case 8: return launch_mst_v<K, SRC, SINK, 5, 0, 256>(L, s);
-      default: return launch_mst_v<K, SRC, SINK, 1, 0>(L, s);
+      default: break;
     }
+    // the GPU holds every ray at once (32 one-warp blocks per SM): dealt by quarter
+    // (60000 / 80000 / 120000 rays 38.6 / 38.8 / 39.7 -> 20.5 / 28.4 / 37.3 ms)
+    if (L.started) return launch_mst_v<K, SRC, SINK, 1, 0, 32>(L, s);
+    // more rays: the queue, with blocks of 64 threads, or of 128 at 51 registers
+    // and a tenth block per SM once the rays are over twice the lanes (300000
+    // rays 82 against 90 ms, 2^20 rays 275 against 272)
+    if (L.n > rays_for(18)) return launch_mst_v<K, SRC, SINK, 10, 0>(L, s);
+    return launch_mst_v<K, SRC, SINK, 1, 0, 64>(L, s);
   } else {
+    // Minkowski's step is a few additions: its constants stay in registers
+    // (16 x 16 pixels 1.10 against 1.17 ms, 256 x 256 2.64 against 2.68)
+    constexpr int F = K == KIND_MINKOWSKI ? FEAT_CHAIN : 0;
     switch (L.variant % 3) {
-      case 1: return launch_mst_v<K, SRC, SINK, 8, 0>(L, s);
-      case 2: return launch_mst_v<K, SRC, SINK, 10, 0>(L, s);
-      default: return launch_mst_v<K, SRC, SINK, 1, 0>(L, s);
+      case 1: return launch_mst_v<K, SRC, SINK, 8, F>(L, s);
+      case 2: return launch_mst_v<K, SRC, SINK, 10, F>(L, s);
+      default: return launch_mst_v<K, SRC, SINK, 1, F>(L, s);
     }
   }
 }

@@ -280,8 +280,8 @@ void geon_set_persistent_reserve_f(double blocks_per_sm);
  * camera rays and ray arrays, 1: equatorial shadow rays). Register cap c: 0 =
  * none, 1 = at most 64 registers per thread, 2 = at most 51. Source 0 takes
  * variant = c (blocks of 128 threads); source 1 takes variant = c + 3 b with
- * block size b: 0 = 128, 1 = 64, 2 = 256 threads. Defaults: 0, for the
- * Schwarzschild equatorial source 2. geon_autotune_mixed times
+ * block size b: 0 = 128, 1 = 64, 2 = 256 threads (source 1,
+ * variant 0: the cap that suits the number of rays). geon_autotune_mixed times
  * every variant on calibration jobs of this metric (n_rays rays - 0 picks four
  * per lane of the widest grid - at most max_steps each; the equatorial job only
  * for Schwarzschild), selects the fastest per source and writes ray-steps/s to
@@ -355,7 +355,7 @@ int geon_shadow_bisect(geon_metric_t schwarzschild, double r_obs, const double* 
                        size_t nb, int iters, double step, int64_t max_steps, int precision,
                        double* alpha_c, double* lo_out, double* hi_out, int64_t* steps_out);
 
-/* Claim order of geon_shadow_classify(_dev) over 65536 rays or more: 1 (the
+/* Claim order of geon_shadow_classify(_dev) over 40000 rays or more: 1 (the
  * default) claims the rays whose impact parameter is at least 0.998 of the
  * critical one (escaping or orbiting near the photon sphere: the long paths)
  * first, so the short ones fill the end of the sweep when lanes run out of
