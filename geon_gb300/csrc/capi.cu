@@ -6,6 +6,7 @@
 
 #include <atomic>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -93,6 +94,56 @@ int sync_and_flags(cudaStream_t s, const int* d_flags, int* h_flags) {
   return GEON_OK;
 }
 
+// Host calls at few points. Each copy from or to pageable memory costs the call
+// ~8 us and each allocation ~2, far more than the kernel's reading and writing, so
+// up to SMALL_CALL bytes go over as one block: [results | flags | a | b] on the
+// device, flags and inputs copied in together, results and flags copied out
+// together (Christoffel symbols at 8 points: 76.0 us as five copies and three
+// allocations, 71.4 as one block).
+// Larger calls copy straight between the caller's arrays and buffers of their own:
+// there a second host copy of the data would cost more than the calls it saves.
+constexpr size_t SMALL_CALL = 16384;
+
+struct SmallCall {
+  DBuf d;
+  cudaStream_t s;
+  size_t out_bytes, a_bytes, b_bytes;
+  alignas(16) char host[SMALL_CALL];
+
+  // (callers form the sizes from at most SMALL_CALL points, so none has wrapped)
+  static bool fits(size_t out, size_t a, size_t b) {
+    return out <= SMALL_CALL && a <= SMALL_CALL && b <= SMALL_CALL &&
+           padded(out) + 8 + padded(a) + padded(b) <= SMALL_CALL;
+  }
+  static size_t padded(size_t bytes) { return (bytes + 7) / 8 * 8; }
+
+  int begin(cudaStream_t st, size_t out, const void* a, size_t an, const void* b, size_t bn) {
+    s = st;
+    out_bytes = padded(out);
+    a_bytes = padded(an);
+    b_bytes = padded(bn);
+    std::memset(host + out_bytes, 0, 8);
+    std::memcpy(host + out_bytes + 8, a, an);
+    if (bn) std::memcpy(host + out_bytes + 8 + a_bytes, b, bn);
+    GEON_CUDA(d.alloc(out_bytes + 8 + a_bytes + b_bytes, s));
+    GEON_CUDA(cudaMemcpyAsync(d.as<char>() + out_bytes, host + out_bytes, 8 + a_bytes + b_bytes, cudaMemcpyHostToDevice, s));
+    return GEON_OK;
+  }
+  template <class T>
+  T* results() const { return reinterpret_cast<T*>(d.as<char>()); }
+  int* flags() const { return reinterpret_cast<int*>(d.as<char>() + out_bytes); }
+  const double* a() const { return reinterpret_cast<const double*>(d.as<char>() + out_bytes + 8); }
+  const double* b() const { return reinterpret_cast<const double*>(d.as<char>() + out_bytes + 8 + a_bytes); }
+  int end(void* out, size_t out_size, int* h_flags) {
+    GEON_CUDA(cudaMemcpyAsync(host, d.p, out_bytes + 8, cudaMemcpyDeviceToHost, s));
+    GEON_CUDA(cudaStreamSynchronize(s));
+    GEON_CUDA(cudaGetLastError());
+    std::memcpy(out, host, out_size);
+    std::memcpy(h_flags, host + out_bytes, sizeof(int));
+    return GEON_OK;
+  }
+};
+
 int singular_status(int flags) {
   if (flags & 1) return fail(GEON_ERR_SINGULAR_METRIC, "metric became singular - coordinate chart broke down");
   return GEON_OK;
@@ -111,14 +162,15 @@ int make_camera(geon_metric_t m, const geon_camera* cam, int64_t spa, CameraDesc
   GEON_CUDA(cudaMemcpyAsync(d_obs, cam->observer, sizeof(double) * 4, cudaMemcpyHostToDevice, s));
   counted();
   GEON_CUDA(launch_tetrad(m->desc, d_obs, d_tet, d_status, s));
-  double tet[16];
+  double back[17];  // the tetrad and, behind it, the status: one copy
   int status = 0;
-  GEON_CUDA(cudaMemcpyAsync(tet, d_tet, sizeof tet, cudaMemcpyDeviceToHost, s));
-  GEON_CUDA(cudaMemcpyAsync(&status, d_status, sizeof status, cudaMemcpyDeviceToHost, s));
+  GEON_CUDA(cudaMemcpyAsync(back, d_tet, sizeof(double) * 16 + sizeof status, cudaMemcpyDeviceToHost, s));
   GEON_CUDA(cudaStreamSynchronize(s));
+  const double* tet = back;
+  std::memcpy(&status, back + 16, sizeof status);
   if (status == GEON_ERR_NOT_TIMELIKE) return fail(status, "observer is not in a timelike region (g_tt >= 0)");
   if (status == GEON_ERR_GRAM_SCHMIDT) return fail(status, "Gram-Schmidt produced non-spacelike vector - chart broken at this point");
-  std::memcpy(c.tet, tet, sizeof tet);
+  std::memcpy(c.tet, tet, sizeof c.tet);
   std::memcpy(c.obs, cam->observer, sizeof c.obs);
   const double fov = cam->fov_y_deg * RADS_PER_DEG;
   const double aspect = (double)cam->width / (double)cam->height;
@@ -554,6 +606,17 @@ static int pointwise(geon_metric_t m, int what, const double* in, size_t n, int 
   if (n == 0) return GEON_OK;
   if (!in || (!out && !iout)) return fail(GEON_ERR_INVALID, "null buffer");
   cudaStream_t s = host_stream();
+  int flags = 0;
+  const size_t small_out = n <= SMALL_CALL ? (out ? sizeof(double) * n * out_width : sizeof(int32_t) * n) : SIZE_MAX;
+  if (n <= SMALL_CALL && SmallCall::fits(small_out, sizeof(double) * n * in_width, 0)) {
+    SmallCall c;
+    if (int rc = c.begin(s, small_out, in, sizeof(double) * n * in_width, nullptr, 0)) return rc;
+    counted();
+    GEON_CUDA(launch_pointwise(m->desc, what, c.a(), (int64_t)n, out ? c.results<double>() : nullptr,
+                               out ? nullptr : c.results<int32_t>(), c.flags(), s));
+    if (int rc = c.end(out ? (void*)out : (void*)iout, small_out, &flags)) return rc;
+    return singular_status(flags);
+  }
   DBuf din, dout, dflags;
   GEON_CUDA(din.alloc(sizeof(double) * n * in_width, s));
   GEON_CUDA(dout.alloc(out ? sizeof(double) * n * out_width : sizeof(int32_t) * n, s));
@@ -565,7 +628,6 @@ static int pointwise(geon_metric_t m, int what, const double* in, size_t n, int 
                              out ? nullptr : dout.as<int32_t>(), dflags.as<int>(), s));
   if (out) GEON_CUDA(cudaMemcpyAsync(out, dout.p, sizeof(double) * n * out_width, cudaMemcpyDeviceToHost, s));
   else GEON_CUDA(cudaMemcpyAsync(iout, dout.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, s));
-  int flags = 0;
   if (int rc = sync_and_flags(s, dflags.as<int>(), &flags)) return rc;
   return singular_status(flags);
 }
@@ -933,8 +995,20 @@ static int curvature_call(geon_metric_t m, int what, const double* x, size_t n, 
   if (n == 0) return GEON_OK;
   if (!x || !out) return fail(GEON_ERR_INVALID, "null buffer");
   cudaStream_t s = host_stream();
-  DBuf dx, dk, dout, dflags;
   const size_t kcount = what == 5 ? (k_shared ? nk : nk * n) : 0;
+  int flags = 0;
+  const bool few = n <= SMALL_CALL && (what != 5 || nk <= SMALL_CALL);
+  if (few && SmallCall::fits(sizeof(double) * n * out_width, sizeof(double) * 4 * n, sizeof(double) * 4 * kcount)) {
+    SmallCall c;
+    if (int rc = c.begin(s, sizeof(double) * n * out_width, x, sizeof(double) * 4 * n, k, sizeof(double) * 4 * kcount))
+      return rc;
+    counted();
+    GEON_CUDA(launch_curvature(m->desc, what, c.a(), (int64_t)n, c.b(), (int64_t)nk, k_shared, c.results<double>(),
+                               c.flags(), s));
+    if (int rc = c.end(out, sizeof(double) * n * out_width, &flags)) return rc;
+    return singular_status(flags);
+  }
+  DBuf dx, dk, dout, dflags;
   GEON_CUDA(dx.alloc(sizeof(double) * 4 * n, s));
   GEON_CUDA(dk.alloc(sizeof(double) * 4 * kcount, s));
   GEON_CUDA(dout.alloc(sizeof(double) * n * out_width, s));
@@ -946,7 +1020,6 @@ static int curvature_call(geon_metric_t m, int what, const double* x, size_t n, 
   GEON_CUDA(launch_curvature(m->desc, what, dx.as<double>(), (int64_t)n, dk.as<double>(), (int64_t)nk,
                              k_shared, dout.as<double>(), dflags.as<int>(), s));
   GEON_CUDA(cudaMemcpyAsync(out, dout.p, sizeof(double) * n * out_width, cudaMemcpyDeviceToHost, s));
-  int flags = 0;
   if (int rc = sync_and_flags(s, dflags.as<int>(), &flags)) return rc;
   return singular_status(flags);
 }
