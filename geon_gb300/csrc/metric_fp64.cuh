@@ -355,13 +355,8 @@ __device__ __forceinline__ void christoffel_schw(const MetricDesc& M, const doub
   G[3 * 16 + 3 * 4 + 2] = cot;
 }
 
-// Generic Christoffel symbols from g^-1 and the FD dg (mod.rs:51-69), dense.
-template <int K>
-__device__ __forceinline__ bool christoffel_generic(const MetricDesc& M, const double x[4], double G[64]) {
-  double ginv[16];
-  const bool ok = metric_g_inv<K>(M, x, ginv);
-  double dg[64];
-  metric_dg<K>(M, x, dg);
+// Generic Christoffel symbols from g^-1 and dg (mod.rs:51-69), dense.
+__device__ __forceinline__ void christoffel_sums(const double ginv[16], const double dg[64], double G[64]) {
 #pragma unroll 1
   for (int mu = 0; mu < 4; ++mu)
 #pragma unroll
@@ -376,6 +371,15 @@ __device__ __forceinline__ bool christoffel_generic(const MetricDesc& M, const d
                 dg[16 * sigma + 4 * alpha + beta]);
         G[16 * mu + 4 * alpha + beta] = 0.5 * s;
       }
+}
+
+template <int K>
+__device__ __forceinline__ bool christoffel_generic(const MetricDesc& M, const double x[4], double G[64]) {
+  double ginv[16];
+  const bool ok = metric_g_inv<K>(M, x, ginv);
+  double dg[64];
+  metric_dg<K>(M, x, dg);
+  christoffel_sums(ginv, dg, G);
   return ok;
 }
 

@@ -435,11 +435,136 @@ __global__ void pointwise_kernel(const MetricDesc M, int what, const double* __r
   }
 }
 
+// ---------------------------------------------------------------------------
+// dg and Christoffel symbols at few points: 8 lanes per point, 4 points per warp.
+// One thread per point is a chain of every metric value the differences need
+// (7 for Alcubierre, 8 for a dense dg), 64-76 cycles per FP64 instruction while
+// its warp is alone on its SM quarter. Here each lane evaluates one of them, the
+// values are exchanged by shuffles, and every lane forms the symbols (the same
+// expressions, so the same bits) and writes an eighth of them.
+// Whole host calls, one thread per point -> 8 lanes (us):
+//                     8 points      608        9728       38912
+//   Alcubierre Gamma  87 -> 33    96 -> 47   130 -> 106  240 -> 274
+//   Alcubierre dg     74 -> 35    96 -> 48   133 -> 95   251 -> 240
+//   Schwarzschild dg  49 -> 33    71 -> 46   107 -> 86   218 -> 202
+//   wormhole Gamma    33 -> 33    50 -> 46    86 -> 84   190 -> 201
+//   sampled Gamma    500 -> 119  570 -> 132  612 -> 465 1200 -> 1720
+// 8 lanes take up to 8 times the FP64 work of a thread's chain, so they win while
+// the chip has quarters to spare: up to FEW_POINTS, 16 warps per SM, for every
+// metric (at 19456 the sampled metric already loses, 640 -> 888).
+// ---------------------------------------------------------------------------
+constexpr int FEW_LANES = 8;
+constexpr int64_t FEW_POINTS = 152 * 64;
+
+__device__ __forceinline__ double of_lane(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane, FEW_LANES); }
+
+__device__ __forceinline__ void shifted(const double x[4], int axis, double h, double y[4]) {
+#pragma unroll
+  for (int a = 0; a < 4; ++a) y[a] = a == axis ? x[a] + h : x[a];
+}
+
+// This lane's metric values at x (lane 0) or one step along an axis g depends on,
+// then all lanes': AXES axes from the first spatial one, in the order +1 -1 +2 ...
+template <int K, int AXES>
+__device__ __forceinline__ void few_values(const MetricDesc& M, const double x[4], int lane, double* gv) {
+  const int axis = lane <= 2 * AXES ? (lane + 1) / 2 : 0;
+  double y[4], a, b;
+  if (axis == 0) shifted(x, 4, 0.0, y);
+  else shifted(x, axis, lane & 1 ? FD_H : -FD_H, y);
+  if (K == KIND_ALCUBIERRE) alc_g00_g01(M, y, &a, &b);
+  else mt_g22_g33(M, y, &a, &b);
+#pragma unroll
+  for (int t = 0; t <= 2 * AXES; ++t) {
+    gv[2 * t] = of_lane(a, t);
+    gv[2 * t + 1] = of_lane(b, t);
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(32) few_points_kernel(const MetricDesc M, int what, const double* __restrict__ in,
+                                                        int64_t n, double* __restrict__ out, int* flags) {
+  const int lane = threadIdx.x % FEW_LANES;
+  const int64_t i = (int64_t)blockIdx.x * (32 / FEW_LANES) + threadIdx.x / FEW_LANES;
+  const bool mine = i < n;  // lanes past the last point repeat it and write nothing
+  const double* xi = in + 4 * (mine ? i : n - 1);
+  const double x[4] = {xi[0], xi[1], xi[2], xi[3]};
+  if (what == PW_CHRISTOFFEL && (K == KIND_ALCUBIERRE || K == KIND_MORRIS_THORNE)) {
+    double gv[14], G[64];
+    bool ok;
+    if (K == KIND_ALCUBIERRE) {
+      few_values<K, 3>(M, x, lane, gv);
+      ok = christoffel_alcubierre_from(gv, G);
+    } else {
+      few_values<K, 2>(M, x, lane, gv);
+      ok = christoffel_morris_thorne_from(gv, G);
+    }
+    if (!mine) return;
+    if (!ok && lane == 0) atomicOr(flags, 1);
+#pragma unroll
+    for (int q = 0; q < 64; ++q)
+      if (q % FEW_LANES == lane) out[64 * i + q] = G[q];
+    return;
+  }
+  // Lanes 2 a and 2 a + 1: g one step forth and back along axis a. The sampled
+  // metric does not depend on t (its t differences are +0); its first pair
+  // evaluates g at x instead.
+  const int axis = lane / 2;
+  double y[4], g[16], d[16];
+  if (K == KIND_FIELD && axis == 0) shifted(x, 4, 0.0, y);
+  else shifted(x, axis, lane & 1 ? -FD_H : FD_H, y);
+  metric_g<K>(M, y, g);
+  const double two_h = 2.0 * FD_H;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const double other = __shfl_xor_sync(0xffffffffu, g[q], 1, FEW_LANES);
+    d[q] = sf::div(lane & 1 ? other - g[q] : g[q] - other, two_h);
+    if (K == KIND_FIELD && axis == 0) d[q] = 0.0;
+  }
+  if (what == PW_DG) {
+    if (!mine) return;
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+      if (q % 2 == (lane & 1)) out[64 * i + 16 * axis + q] = d[q];
+    return;
+  }
+  if (K == KIND_FIELD) {
+    double at[16], gi[16], dg[64], G[64];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) at[q] = of_lane(g[q], 0);
+#pragma unroll
+    for (int q = 0; q < 64; ++q) dg[q] = of_lane(d[q % 16], 2 * (q / 16));
+    const bool ok = inv4(at, gi);
+    christoffel_sums(gi, dg, G);
+    if (!mine) return;
+    if (!ok && lane == 0) atomicOr(flags, 1);
+#pragma unroll
+    for (int q = 0; q < 64; ++q)
+      if (q % FEW_LANES == lane) out[64 * i + q] = G[q];
+  }
+}
+
+// Whether a call differentiates g (the others are one evaluation per point).
+bool few_differences(int kind, int what) {
+  if (what == PW_DG) return kind != KIND_MINKOWSKI;
+  return what == PW_CHRISTOFFEL && (kind == KIND_ALCUBIERRE || kind == KIND_MORRIS_THORNE || kind == KIND_FIELD);
+}
+
 cudaError_t launch_pointwise(const MetricDesc& M, int what, const double* in, int64_t n, double* out,
                              int32_t* iout, int* flags, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   const int block = 128;
   const unsigned grid = (unsigned)((n + block - 1) / block);
+  if (n <= FEW_POINTS && few_differences(M.kind, what)) {
+    const unsigned few = (unsigned)((n + 32 / FEW_LANES - 1) / (32 / FEW_LANES));
+    switch (M.kind) {
+      case KIND_SCHWARZSCHILD: few_points_kernel<KIND_SCHWARZSCHILD><<<few, 32, 0, s>>>(M, what, in, n, out, flags); break;
+      case KIND_ALCUBIERRE: few_points_kernel<KIND_ALCUBIERRE><<<few, 32, 0, s>>>(M, what, in, n, out, flags); break;
+      case KIND_MORRIS_THORNE: few_points_kernel<KIND_MORRIS_THORNE><<<few, 32, 0, s>>>(M, what, in, n, out, flags); break;
+      case KIND_FIELD: few_points_kernel<KIND_FIELD><<<few, 32, 0, s>>>(M, what, in, n, out, flags); break;
+      default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+  }
   switch (M.kind) {
     case KIND_MINKOWSKI: pointwise_kernel<KIND_MINKOWSKI><<<grid, block, 0, s>>>(M, what, in, n, out, iout, flags); break;
     case KIND_SCHWARZSCHILD: pointwise_kernel<KIND_SCHWARZSCHILD><<<grid, block, 0, s>>>(M, what, in, n, out, iout, flags); break;
