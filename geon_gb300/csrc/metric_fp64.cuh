@@ -223,11 +223,11 @@ __device__ __forceinline__ void metric_g(const MetricDesc& M, const double x[4],
     g[0] = -1.0; g[5] = 1.0; g[10] = 1.0; g[15] = 1.0;
   } else if (K == KIND_SCHWARZSCHILD) {  // schwarzschild.rs:33-45
     const double r = x[1], theta = x[2], m = M.p[0];
-    const double f = 1.0 - 2.0 * m / r;
+    const double f = 1.0 - sf::div(2.0 * m, r);
     double sin_t, cos_t;
     dm::sincos_det(theta, &sin_t, &cos_t);
     g[0] = -f;
-    g[5] = 1.0 / f;
+    g[5] = sf::rcp(f);
     g[10] = r * r;
     g[15] = r * r * sin_t * sin_t;
   } else if (K == KIND_ALCUBIERRE) {  // alcubierre.rs:33-63
@@ -446,8 +446,8 @@ __device__ __forceinline__ void metric_asymptotic_direction(const MetricDesc& M,
                                                             const double p[4], double out[3]) {
   if (K == KIND_ALCUBIERRE || (K == KIND_FIELD && M.f.chart == GEON_CHART_CARTESIAN)) {
     const double vx = p[1], vy = p[2], vz = p[3];
-    const double n = fmax(sqrt(vx * vx + vy * vy + vz * vz), 1e-30);
-    out[0] = vx / n; out[1] = vy / n; out[2] = vz / n;
+    const double n = fmax(sf::root(vx * vx + vy * vy + vz * vz), 1e-30);
+    out[0] = sf::div(vx, n); out[1] = sf::div(vy, n); out[2] = sf::div(vz, n);
     return;
   }
   double sin_t, cos_t, sin_p, cos_p;
@@ -460,16 +460,16 @@ __device__ __forceinline__ void metric_asymptotic_direction(const MetricDesc& M,
     const double vx = sin_t * cos_p * pr + r_eff * cos_t * cos_p * pt - r_eff * sin_t * sin_p * pp;
     const double vy = sin_t * sin_p * pr + r_eff * cos_t * sin_p * pt + r_eff * sin_t * cos_p * pp;
     const double vz = cos_t * pr - r_eff * sin_t * pt;
-    const double n = fmax(sqrt(vx * vx + vy * vy + vz * vz), 1e-30);
+    const double n = fmax(sf::root(vx * vx + vy * vy + vz * vz), 1e-30);
     const double sign = l < 0.0 ? -1.0 : 1.0;
-    out[0] = sign * vx / n; out[1] = vy / n; out[2] = vz / n;
+    out[0] = sf::div(sign * vx, n); out[1] = sf::div(vy, n); out[2] = sf::div(vz, n);
   } else {
     const double r = x[1];
     const double vx = sin_t * cos_p * pr + r * cos_t * cos_p * pt - r * sin_t * sin_p * pp;
     const double vy = sin_t * sin_p * pr + r * cos_t * sin_p * pt + r * sin_t * cos_p * pp;
     const double vz = cos_t * pr - r * sin_t * pt;
-    const double n = fmax(sqrt(vx * vx + vy * vy + vz * vz), 1e-30);
-    out[0] = vx / n; out[1] = vy / n; out[2] = vz / n;
+    const double n = fmax(sf::root(vx * vx + vy * vy + vz * vz), 1e-30);
+    out[0] = sf::div(vx, n); out[1] = sf::div(vy, n); out[2] = sf::div(vz, n);
   }
 }
 
@@ -662,13 +662,29 @@ __device__ __forceinline__ bool rk4_step_schw_soft(const MetricDesc& M, const do
   return worst < sf::RANGE - (2u << 21);  // h itself is twice half_h
 }
 
-// Residual |g(p, p)| at the position of y (geodesic.rs:82-84), dense dot4.
+// Entries of g that the metric fixes at zero.
+template <int K>
+__host__ __device__ constexpr bool entry_is_zero(int i, int j) {
+  if (K == KIND_FIELD || i == j) return false;
+  return !(K == KIND_ALCUBIERRE && i + j == 1);
+}
+
+// Residual |g(p, p)| at the position of y (geodesic.rs:82-84): dot4 in its
+// order. With finite p the terms of zero entries are zeros and leave the sum,
+// which starts at +0, as it is.
 template <int K>
 __device__ __forceinline__ double null_residual(const MetricDesc& M, const double y[8]) {
   double g[16];
   metric_g<K>(M, y, g);
   const double p[4] = {y[4], y[5], y[6], y[7]};
-  return fabs(dot4(g, p, p));
+  if (!(sf::finite(p[0]) && sf::finite(p[1]) && sf::finite(p[2]) && sf::finite(p[3]))) return fabs(dot4(g, p, p));
+  double s = 0.0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (!entry_is_zero<K>(i, j)) s += g[4 * i + j] * p[i] * p[j];
+  return fabs(s);
 }
 
 }  // namespace geon

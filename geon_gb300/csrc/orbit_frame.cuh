@@ -3,11 +3,22 @@
 // device code (the CPU tests compile it with g++).
 #pragma once
 #include <math.h>
+#ifdef __CUDACC__
+#include "softfp.cuh"
+#endif
 
 #ifdef __CUDACC__
 #define GEON_HD __host__ __device__
 #else
 #define GEON_HD
+#endif
+// Division and square root: in the integer pipes on the device (the same bits).
+#ifdef __CUDA_ARCH__
+#define GEON_DIV(a, b) sf::div(a, b)
+#define GEON_ROOT(a) sf::root(a)
+#else
+#define GEON_DIV(a, b) ((a) / (b))
+#define GEON_ROOT(a) ::sqrt(a)
 #endif
 
 namespace geon {
@@ -49,8 +60,8 @@ GEON_HD inline void orbit_out(const double yr[8], const float e1[3], const float
     n[i] = cf * (double)e1[i] + sf * (double)e2[i];
     w[i] = yr[7] * (cf * (double)e2[i] - sf * (double)e1[i]);
   }
-  const double nn = ::sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-  const double nz = ::fmin(1.0, ::fmax(-1.0, n[2] / nn));
+  const double nn = GEON_ROOT(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+  const double nz = ::fmin(1.0, ::fmax(-1.0, GEON_DIV(n[2], nn)));
   const double th = ::acos(nz), ph = ::atan2(n[1], n[0]);
   double st, ct, sp, cp;
   ::sincos(th, &st, &ct);
@@ -58,7 +69,7 @@ GEON_HD inline void orbit_out(const double yr[8], const float e1[3], const float
   y[0] = yr[0]; y[1] = yr[1]; y[2] = th; y[3] = ph;
   y[4] = yr[4]; y[5] = yr[5];
   y[6] = w[0] * ct * cp + w[1] * ct * sp - w[2] * st;
-  y[7] = (w[1] * cp - w[0] * sp) / st;
+  y[7] = GEON_DIV(w[1] * cp - w[0] * sp, st);
 }
 
 }  // namespace geon

@@ -37,8 +37,11 @@ __device__ __forceinline__ int64_t sky_to_i64(double v) {
   return (int64_t)v;
 }
 
+// Within two divisors of zero, where every finite angle lies, the remainder is a
+// itself or one exact subtraction.
 __device__ __forceinline__ double sky_rem_euclid(double a, double b) {
-  const double r = fmod(a, b);
+  const double mag = fabs(a);
+  const double r = mag < b ? a : (mag < 2.0 * b ? copysign(mag - b, a) : fmod(a, b));
   return r < 0.0 ? r + fabs(b) : r;
 }
 
@@ -53,34 +56,38 @@ __device__ __forceinline__ double sky_clamp(double x, double lo, double hi) {
   return x;
 }
 
+// In global memory: as a local array it is 144 bytes of stack that every thread
+// writes before it reads three of them.
+static __device__ const double SKY_PALETTE[6][3] = {{0.15, 0.08, 0.20}, {0.08, 0.15, 0.22}, {0.20, 0.15, 0.08},
+                                                    {0.10, 0.18, 0.10}, {0.22, 0.10, 0.10}, {0.10, 0.10, 0.22}};
+
 __device__ __forceinline__ void sky_sample(const double dir[3], bool show_stars, float out[3]) {
   const double x = dir[0], y = dir[1], z = dir[2];
-  const double r = fmax(sqrt(x * x + y * y + z * z), 1e-30);
-  const double theta = acos(sky_clamp(z / r, -1.0, 1.0));
+  const double r = fmax(sf::root(x * x + y * y + z * z), 1e-30);
+  const double theta = acos(sky_clamp(sf::div(z, r), -1.0, 1.0));
   const double phi = atan2(y, x);
   const double phi_shift = sky_rem_euclid(phi + SKY_PHI_OFFSET, SKY_TAU);
   const double theta_shift = sky_clamp(theta + SKY_THETA_OFFSET, 0.0, SKY_PI);
+  const double u = sf::div(phi_shift, SKY_TAU), v = sf::div(theta_shift, SKY_PI);
   // sectors (sky.rs:72-104)
-  const int64_t phi_mod = sky_to_i64(floor(phi_shift / SKY_TAU * 6.0));
-  const int64_t band = sky_to_i64(floor(theta_shift / SKY_PI * 3.0));
-  const double pal[6][3] = {{0.15, 0.08, 0.20}, {0.08, 0.15, 0.22}, {0.20, 0.15, 0.08},
-                            {0.10, 0.18, 0.10}, {0.22, 0.10, 0.10}, {0.10, 0.10, 0.22}};
+  const int64_t phi_mod = sky_to_i64(floor(u * 6.0));
+  const int64_t band = sky_to_i64(floor(v * 3.0));
   const int sector = (int)sky_rem_euclid_i(phi_mod, 6);
   const double band_mod = sky_rem_euclid_i(band, 2) == 0 ? 1.0 : 0.6;
-  const int64_t ic = sky_to_i64(floor(phi_shift / SKY_TAU * 24.0));
-  const int64_t jc = sky_to_i64(floor(theta_shift / SKY_PI * 12.0));
+  const int64_t ic = sky_to_i64(floor(u * 24.0));
+  const int64_t jc = sky_to_i64(floor(v * 12.0));
   const double check = sky_rem_euclid_i(ic + jc, 2) == 0 ? 1.0 : 0.55;
-  float s0 = (float)(pal[sector][0] * band_mod * check);
-  float s1 = (float)(pal[sector][1] * band_mod * check);
-  float s2 = (float)(pal[sector][2] * band_mod * check);
+  float s0 = (float)(SKY_PALETTE[sector][0] * band_mod * check);
+  float s1 = (float)(SKY_PALETTE[sector][1] * band_mod * check);
+  float s2 = (float)(SKY_PALETTE[sector][2] * band_mod * check);
   // stars (sky.rs:43-68)
   float t0 = 0.0f, t1 = 0.0f, t2 = 0.0f;
   if (show_stars) {
-    const int64_t i = sky_to_i64(floor(phi_shift / SKY_TAU * 512.0));
-    const int64_t j = sky_to_i64(floor(theta_shift / SKY_PI * 256.0));
+    const int64_t i = sky_to_i64(floor(u * 512.0));
+    const int64_t j = sky_to_i64(floor(v * 256.0));
     const uint64_t h = sky_hash2(i, j);
-    const double prob = (double)(h & 0xFFFF) / 65535.0;
-    if (prob < 0.004) {
+    // (h & 0xFFFF) / 65535 < 0.004, over whole numbers
+    if ((h & 0xFFFF) <= 262) {
       const double brightness = 0.4 + 0.6 * ((double)((h >> 16) & 0xFF) / 255.0);
       const double temp = (double)((h >> 24) & 0xFF) / 255.0;
       t0 = (float)(brightness * (1.0 - 0.3 * temp));
