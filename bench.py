@@ -742,7 +742,9 @@ def config3_leg(geon, lib, n, row_step, check_agreeing=256, peak32=None, peak64=
                           f"{c['metric_eval_flops_per_rhs']} for the metric at {c['metric_points_per_rhs']} "
                           f"distinct points, x4, + {104} RK4 combine; not counted: {c['calls_per_step']} per step",
             "achieved": o["fp64_ray_steps_per_s"] * c["flops_per_step"] / 1e12, "unit": "TFLOP/s",
-            "sample": f"{rays} rays ({(rays + 127) // 128} blocks of 128 on the GPU), host API wall time"}
+            "note": "Alcubierre rays in flat space take whole groups of steps as position additions (same bits), so the "
+                    "work counted per ray-step is not done for most of them and frac can exceed 1",
+            "sample": f"{rays} rays (one-warp blocks on the GPU), host API wall time"}
         o["roofline_mixed"] = {
             "bound": "fp32 pipe", "alg_flops_per_ray_step": MIXED_CLOSED_FORM_FLOPS_PER_STEP[name],
             "definition": "the mixed path's closed-form right-hand side (metric_analytic.cuh; transcendental "
@@ -864,8 +866,10 @@ def config4_leg(geon, n, peak64, cpu_budget_s=3.0):
             "host_api_ms_fresh_arrays": 1e3 * dt_fresh, "host_api_same_bits": host_same, "kernel_ms": kernel_ms,
             "kernel_points_per_s": len(pts) / (1e-3 * kernel_ms),
             "roofline": {"bound": "fp64 pipe", "achieved": ach, "peak": peak64, "unit": "TFLOP/s",
-                         "frac": ach / peak64 if peak64 else None, "kernel": "curvature_grid_kernel<Alcubierre>",
+                         "frac": ach / peak64 if peak64 else None, "kernel": "curvature_point_kernel<Alcubierre, grid>",
                          "alg_flops_per_point": CURV_FLOPS_PER_POINT,
+                         "note": "flops of the reference's dense algorithm; the kernel forms the nonzero terms only, "
+                                 "so frac can exceed 1",
                          "hbm_gbs": len(pts) * (16 + 16) * 8 / (kernel_ms / 1e3) / 1e9},
             "device_api_same_bits": dev_same, "bit_exact_vs_oracle_geon_sample": bit_exact,
             "bit_exact_vs_oracle_libm_sample": bit_exact_libm,

@@ -16,7 +16,9 @@ CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_lib", "autotu
 CAPS = ("no register cap", "<=64 registers", "<=51 registers")
 BLOCKS = (128, 64, 256)
 # source 0 (camera rays, ray arrays): the register caps at 128 threads per block;
-# source 1 (equatorial shadow rays): cap + 3 * block-size index
+# source 1 (equatorial shadow rays): cap + 3 * block-size index. Its variant 0,
+# the default, picks cap and block by the number of rays; the calibration runs it
+# as one candidate at its own number of rays.
 VARIANTS = tuple(f"{c}, {b} threads/block" for b in BLOCKS for c in CAPS)
 
 
