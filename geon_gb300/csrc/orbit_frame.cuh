@@ -38,11 +38,11 @@ GEON_HD inline void orbit_in(const double y[8], double yr[8], float e1[3], float
   const double ep[3] = {-sp, cp, 0.0};
   double w[3];
   for (int i = 0; i < 3; ++i) w[i] = y[6] * et[i] + y[7] * st * ep[i];
-  const double wn = ::sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
+  const double wn = GEON_ROOT(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
   const bool turning = wn > 0.0 && wn < INFINITY;
   for (int i = 0; i < 3; ++i) {
     e1[i] = (float)n[i];
-    e2[i] = (float)(turning ? w[i] / wn : et[i]);
+    e2[i] = (float)(turning ? GEON_DIV(w[i], wn) : et[i]);
   }
   yr[0] = y[0]; yr[1] = y[1]; yr[2] = 1.5707963267948966; yr[3] = 0.0;
   yr[4] = y[4]; yr[5] = y[5]; yr[6] = 0.0; yr[7] = turning ? wn : 0.0;
