@@ -1057,7 +1057,7 @@ __global__ void __launch_bounds__(128) render_prepare_kernel(const TraceLaunch L
 // g in the residual, and the sky's palette in memory instead of 144 bytes of
 // stack written by every thread. A 960x540 frame at 2x2 samples (2.07 million
 // samples): whole render 26.85 -> 26.33 ms, the kernel being 3.2 of the first
-(25.83 with the camera ray and the orbit frame, formed again here, done so too).
+// (25.83 with the camera ray and the orbit frame, formed again here, done so too).
 template <int K, int FEAT>
 __global__ void __launch_bounds__(128) render_shade_kernel(const TraceLaunch L) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
