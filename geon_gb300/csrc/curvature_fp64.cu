@@ -432,9 +432,11 @@ curvature_kernel(const MetricDesc M, int what, const double* __restrict__ xs, in
 // shared memory (one column per thread), the distinct nonzero symbols slot by
 // slot, their differences, the sparse Ricci tensor, and the vectors of the point
 // one after another. Terms that are structurally zero, or the difference of two
-// equal values, are left out, so finite results have the dense code's bits up
-// to the sign of a zero; a point with a singular metric or a non-finite symbol
-// goes through the dense sums (dense_ricci), which treat it as before.
+// equal values, are left out. Such a term of the dense sums is a zero while
+// nothing overflows, so results have the dense code's bits up to the sign of a
+// zero where every symbol is below SYMBOL_BOUND; a point with a singular metric
+// or a larger or non-finite symbol goes through the dense sums (dense_ricci),
+// where 0 * inf and inf - inf are NaN as they are in the reference.
 // Divisions and square roots run in the integer pipes (softfp.cuh), and so do
 // the tests and the conversion of the random directions. Still bound by the FP64
 // pipe, with about 4400 instead of 10400 FP64 operations per Alcubierre point
@@ -442,6 +444,9 @@ curvature_kernel(const MetricDesc M, int what, const double* __restrict__ xs, in
 // 32736 Morris-Thorne points 518 -> 170 us, 10^5 Schwarzschild scalars 486 -> 90 us.
 // ---------------------------------------------------------------------------
 constexpr int POINT_THREADS = 64;
+// High word of 2^500. Below it products of two symbols stay below 2^1000, their
+// differences over 2 h below 2^518, and the sums of a Riemann entry finite.
+constexpr unsigned SYMBOL_BOUND = (1023u + 500u) << 20;
 
 // Ricci tensor of one point by the dense sums of curvature.rs:48-85.
 template <int K>
@@ -712,7 +717,7 @@ curvature_point_kernel(const MetricDesc M, int what, const double* __restrict__ 
     }
   }
   double ric[16];
-  const bool plain = regular && big < 2u * 0x7ff00000u;
+  const bool plain = regular && big < 2u * SYMBOL_BOUND;
   if (plain) {
     PM::ricci(c, [&](int axis, int i) { return diff[(axis * PM::ND + PM::diff_place(i)) * POINT_THREADS]; }, ric);
   } else {
