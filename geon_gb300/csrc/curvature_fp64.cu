@@ -640,8 +640,26 @@ struct PointMetric<KIND_SCHWARZSCHILD> {
   }
 };
 
+// T(k, k) of a point's generated vectors with the dense Gram-Schmidt and sums.
+__device__ __noinline__ void dense_contractions(const double* g, const double* t, uint64_t seed, int64_t pt, int64_t nk,
+                                                double* nec, double* kout) {
+  double tet[16];
+  const bool ok = point_tetrad(g, tet);
+  for (int64_t q = 0; q < nk; ++q) {
+    double k[4];
+    point_null_vector(tet, ok, seed, pt, nk, q, k);
+    double sacc = 0.0;
+    for (int mu = 0; mu < 4; ++mu) {
+      if (kout) kout[4 * (pt * nk + q) + mu] = k[mu];
+      for (int nu = 0; nu < 4; ++nu) sacc += t[4 * mu + nu] * k[mu] * k[nu];
+    }
+    nec[pt * nk + q] = sacc;
+  }
+}
+
 // The static observer's tetrad of a point (point_tetrad) with the zero terms of
-// the Gram-Schmidt sums left out: e0 = a d_t, e1 = (b, c, 0, 0), e2 and e3 along
+// the Gram-Schmidt sums left out, for points whose symbols are below SYMBOL_BOUND
+// (g is finite there; an infinite entry makes 0 * inf of the terms left out): e0 = a d_t, e1 = (b, c, 0, 0), e2 and e3 along
 // their axes. Diagonal metrics have b = 0.
 struct SparseTetrad {
   double a, b, c, e2, e3;
@@ -762,6 +780,10 @@ curvature_point_kernel(const MetricDesc M, int what, const double* __restrict__ 
   double t[16];
 #pragma unroll
   for (int q = 0; q < 16; ++q) t[q] = ein[q] * factor;  // curvature.rs:112-122
+  if (what == 6 && !plain) {
+    dense_contractions(g, t, seed, pt, nk, out2, kout);
+    return;
+  }
   SparseTetrad tet = {};
   if (what == 6) tet = sparse_tetrad<K>(g);
   // T(k, k) (curvature.rs:127-136) of the point's vectors, one after another
