@@ -305,7 +305,8 @@ def main():
     ap.add_argument("--fp64-sample", type=int, default=32, help="accuracy and FP64 legs trace every k-th sweep ray")
     ap.add_argument("--fp64-steps", type=int, default=3, help="timed steps of the FP64 latency leg")
     ap.add_argument("--variant", type=int, default=-1,
-                    help="mixed equatorial kernel variant (register cap + 3 x block size index); -1: the autotuner's")
+                    help="mixed equatorial kernel variant (register cap + 3 x block size index, 9: by the number of rays); "
+                         "-1: the autotuner's")
     ap.add_argument("--sweep-order", type=int, default=1, help="longest-first claim order of the sweep (1) or not (0)")
     ap.add_argument("--legs", default="all",
                     help="comma list of legs beside the headline (accuracy,fp64,e2e,cpu,config1,config3,config4,"
@@ -440,7 +441,7 @@ def main():
                                 else f"bisections beside the sweep, {args.reserve} block slots per SM reserved"),
                    "bisect_rays_per_round": args.bisect_rays,
                    "mixed_kernel_variant": lib.geon_get_mixed_variant(1, 1) if prec == 1 else None,
-                   "mixed_block_size": (128, 64, 256)[lib.geon_get_mixed_variant(1, 1) // 3] if prec == 1 else None,
+                   "mixed_block_size": geon.autotune.block_size(lib.geon_get_mixed_variant(1, 1)) if prec == 1 else None,
                    "sweep_claim_order": "longest first" if args.sweep_order else "index order",
                    "autotune_rates": None if tuned is None else tuned.get("rates")},
         "latency": {"step_ms_p50": pct(times, 50), "step_ms_p99": pct(times, 99),

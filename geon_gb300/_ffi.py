@@ -135,6 +135,8 @@ SIGNATURES = {
     "geon_set_persistent_reserve_f": (None, [ctypes.c_double]),
     "geon_set_mixed_variant": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "geon_get_mixed_variant": (ctypes.c_int, [ctypes.c_int, ctypes.c_int]),
+    "geon_set_sweep_variant_above": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int64]),
+    "geon_get_sweep_variant_above": (ctypes.c_int64, [ctypes.c_int]),
     "geon_autotune_mixed": (ctypes.c_int, [c_void_p, ctypes.c_int64, ctypes.c_int64, c_double_p,
                                            ctypes.POINTER(ctypes.c_int)]),
     "geon_riemann": (ctypes.c_int, [c_void_p, c_double_p, c_size_t, c_double_p]),

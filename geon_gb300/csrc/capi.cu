@@ -4,6 +4,7 @@
 // -ffp-contract=off.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdint>
@@ -36,9 +37,10 @@ std::atomic<int> g_sweep_order{1};  // longest-first claim order of shadow sweep
 std::atomic<float> g_reserve{0.0f};
 std::atomic<double> g_rtol{1e-10};  // GEON_ADAPTIVE error tolerances
 std::atomic<double> g_atol{1e-12};
-// Mixed-kernel variant per metric kind and ray source (camera/array, equatorial),
-// chosen by geon_autotune_mixed (default 0).
-std::atomic<int> g_variant[4][2] = {{{0}, {0}}, {{0}, {0}}, {{0}, {0}}, {{0}, {0}}};
+// Mixed-kernel variant per metric kind of camera rays and ray arrays, and of
+// equatorial rays (sweep_choice), set by the caller or by geon_autotune_mixed.
+std::atomic<int> g_variant[4] = {{0}, {0}, {0}, {0}};
+std::atomic<int64_t> g_sweep[4] = {{SWEEP_BY_SIZE}, {SWEEP_BY_SIZE}, {SWEEP_BY_SIZE}, {SWEEP_BY_SIZE}};
 // Kernels launched by this library since load (ours only; memsets excluded).
 std::atomic<unsigned long long> g_launches{0};
 inline void counted(unsigned long long n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
@@ -231,7 +233,7 @@ TraceLaunch base_launch(geon_metric_t m, double step, int64_t max_steps) {
   L.mixed_flags = (g_reproject.load() ? MIXED_REPROJECT : 0) | (g_orbit.load() ? MIXED_ORBIT : 0) |
                   (g_nullfix.load() ? MIXED_NULLFIX : 0);
   L.reserve_per_sm = g_reserve.load();
-  L.variant = g_variant[m->desc.kind][0].load();
+  L.variant = g_variant[m->desc.kind].load();
   L.rtol = g_rtol.load();
   L.atol = g_atol.load();
   return L;
@@ -240,7 +242,7 @@ TraceLaunch base_launch(geon_metric_t m, double step, int64_t max_steps) {
 cudaError_t launch_trace(const TraceLaunch& L0, int precision, int src, int sink, cudaStream_t s) {
   if (L0.n > 0) counted();
   TraceLaunch L = L0;
-  if (src == SRC_EQUATORIAL) L.variant = g_variant[L.M.kind][1].load();
+  if (src == SRC_EQUATORIAL) L.variant = sweep_variant(g_sweep[L.M.kind].load(), L.n);
   if (precision == GEON_MIXED) return launch_trace_mixed(L, src, sink, s);
   if (precision == GEON_ADAPTIVE) return launch_trace_adaptive(L, src, sink, s);
   if (precision == GEON_FP64_FAST) return launch_trace_fp64fast(L, src, sink, s);
@@ -374,15 +376,29 @@ void geon_set_persistent_reserve_f(double blocks_per_sm) {
 
 int geon_set_mixed_variant(int kind, int source, int variant) {
   if (kind < GEON_MINKOWSKI || kind > GEON_MORRIS_THORNE || source < 0 || source > 1 || variant < 0 ||
-      variant >= (source == 1 ? MIXED_VARIANTS : MIXED_CAPS))
+      variant >= (source == 1 ? SWEEP_BY_SIZE + 1 : MIXED_CAPS))
     return fail(GEON_ERR_INVALID, "bad kind, source or variant");
-  g_variant[kind][source].store(variant);
+  if (source == 1) g_sweep[kind].store(sweep_choice(variant, 0));
+  else g_variant[kind].store(variant);
+  return GEON_OK;
+}
+
+int geon_set_sweep_variant_above(int kind, int variant, int64_t rays) {
+  if (kind < GEON_MINKOWSKI || kind > GEON_MORRIS_THORNE || variant < 0 || variant > SWEEP_BY_SIZE || rays < 0 ||
+      rays >= (int64_t)1 << 58)
+    return fail(GEON_ERR_INVALID, "bad kind, variant or number of rays");
+  g_sweep[kind].store(sweep_choice(variant, rays));
   return GEON_OK;
 }
 
 int geon_get_mixed_variant(int kind, int source) {
   if (kind < GEON_MINKOWSKI || kind > GEON_MORRIS_THORNE || source < 0 || source > 1) return GEON_ERR_INVALID;
-  return g_variant[kind][source].load();
+  return source == 1 ? sweep_choice_variant(g_sweep[kind].load()) : g_variant[kind].load();
+}
+
+int64_t geon_get_sweep_variant_above(int kind) {
+  if (kind < GEON_MINKOWSKI || kind > GEON_MORRIS_THORNE) return GEON_ERR_INVALID;
+  return g_sweep[kind].load() >> 4;
 }
 
 // Autotuner: time every register-cap variant of the mixed kernel on calibration
@@ -395,14 +411,12 @@ int geon_get_mixed_variant(int kind, int source) {
 // Every ray is capped at max_steps. rates_out[3 + 9] receives ray-steps/s per
 // (source, variant): 3 register caps for source 0, then 9 (cap + 3 x block size
 // 128/64/256) for source 1; best_out[2] the chosen variant per source (-1: not
-// tuned).
+// tuned; SWEEP_BY_SIZE: source 1 keeps the rule, sweep_tuned).
 static int time_variants(const TraceLaunch& base, int src, int sink, int64_t n, const int64_t* d_steps,
-                         cudaStream_t s, double* rates, int* best, int nvariants) {
+                         cudaStream_t s, double* rates, int nvariants) {
   cudaEvent_t a, b;
   GEON_CUDA(cudaEventCreate(&a));
   GEON_CUDA(cudaEventCreate(&b));
-  double best_rate = -1.0;
-  *best = 0;
   std::vector<int64_t> st(n);
   for (int v = 0; v < nvariants; ++v) {
     TraceLaunch L = base;
@@ -426,12 +440,7 @@ static int time_variants(const TraceLaunch& base, int src, int sink, int64_t n, 
     GEON_CUDA(cudaMemcpy(st.data(), d_steps, sizeof(int64_t) * n, cudaMemcpyDeviceToHost));
     double total = 0.0;
     for (int64_t q = 0; q < n; ++q) total += (double)st[q];
-    const double rate = total / (best_ms * 1e-3);
-    rates[v] = rate;
-    if (rate > best_rate) {
-      best_rate = rate;
-      *best = v;
-    }
+    rates[v] = total / (best_ms * 1e-3);
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
@@ -442,16 +451,16 @@ int geon_autotune_mixed(geon_metric_t m, int64_t n_rays, int64_t max_steps, doub
   if (int rc = check_metric(m)) return rc;
   if (m->desc.kind == GEON_FIELD) return fail(GEON_ERR_UNSUPPORTED, "no mixed-precision stepper for a sampled metric");
   if (n_rays < 0 || max_steps <= 0) return fail(GEON_ERR_INVALID, "bad calibration size");
+  int dev = 0, sms = 0;
+  GEON_CUDA(cudaGetDevice(&dev));
+  GEON_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (n_rays == 0) {
     // four rays per lane of the largest variant's grid: occupancy decides the
     // rate only when every lane has work for most of the launch
-    int dev = 0, sms = 0;
-    GEON_CUDA(cudaGetDevice(&dev));
-    GEON_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     n_rays = (int64_t)sms * 6 * 128 * 4;  // 128 threads per trace block
   }
   const int kind = m->desc.kind;
-  double rates[MIXED_CAPS + MIXED_VARIANTS] = {};
+  double rates[MIXED_CAPS + SWEEP_VARIANTS] = {};
   int best[2] = {0, -1};
   cudaStream_t s = host_stream();
   geon_camera cam;
@@ -485,9 +494,10 @@ int geon_autotune_mixed(geon_metric_t m, int64_t n_rays, int64_t max_steps, doub
   L.flags = reinterpret_cast<int*>(L.queue + 1);
   L.ystate = dstate.as<uint32_t>();
   // the trace kernel of the three-kernel render (camera rays prepared, states out)
-  if (int rc = time_variants(L, SRC_STATE, SINK_STATE, n, dsteps.as<int64_t>(), s, rates, &best[0], MIXED_CAPS))
+  if (int rc = time_variants(L, SRC_STATE, SINK_STATE, n, dsteps.as<int64_t>(), s, rates, MIXED_CAPS))
     return rc;
-  g_variant[kind][0].store(best[0]);
+  best[0] = (int)(std::max_element(rates, rates + MIXED_CAPS) - rates);
+  g_variant[kind].store(best[0]);
   if (kind == GEON_SCHWARZSCHILD) {
     std::vector<double> alpha(n);
     for (int64_t i = 0; i < n; ++i) alpha[i] = (10.0 + 10.0 * ((double)((i * 7919) % n) + 0.5) / (double)n) * RADS_PER_DEG;
@@ -502,9 +512,11 @@ int geon_autotune_mixed(geon_metric_t m, int64_t n_rays, int64_t max_steps, doub
     E.queue = ws.as<unsigned long long>();
     E.flags = reinterpret_cast<int*>(E.queue + 1);
     if (int rc = time_variants(E, SRC_EQUATORIAL, SINK_SHADOW, n, dsteps.as<int64_t>(), s, rates + MIXED_CAPS,
-                               &best[1], MIXED_VARIANTS))
+                               SWEEP_VARIANTS))
       return rc;
-    g_variant[kind][1].store(best[1]);
+    const int64_t choice = sweep_tuned(rates + MIXED_CAPS, n, sms);
+    g_sweep[kind].store(choice);
+    best[1] = sweep_choice_variant(choice);
   }
   if (rates_out) std::memcpy(rates_out, rates, sizeof rates);
   if (best_out) {
@@ -1076,9 +1088,9 @@ static int classify_dev(geon_metric_t m, double r_obs, const double* d_alpha, in
   int dev = 0, sms = 0;
   GEON_CUDA(cudaGetDevice(&dev));
   GEON_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const bool resident = precision == GEON_MIXED && n > (int64_t)sms * 128 && n <= (int64_t)sms * 1024 &&
-                        4u * (unsigned)sms < RESIDENT_QUARTERS && g_variant[m->desc.kind][1].load() == 0 &&
-                        g_reserve.load() == 0.0f;
+  const bool resident = precision == GEON_MIXED && n > sweep_one_warp(sms) && n <= sweep_held(sms) &&
+                        4u * (unsigned)sms < RESIDENT_QUARTERS &&
+                        sweep_variant(g_sweep[m->desc.kind].load(), n) == SWEEP_BY_SIZE && g_reserve.load() == 0.0f;
   const size_t ws_bytes = sizeof(unsigned long long) * 4 +
                           (resident ? sizeof(unsigned) * (RESIDENT_QUARTERS + (size_t)(n + 31) / 32) : 0);
   GEON_CUDA(ws.alloc(ws_bytes, s));

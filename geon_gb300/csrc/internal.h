@@ -6,6 +6,7 @@
 #include <string>
 
 #include "../../include/geon_gpu.h"
+#include "sweep_rule.h"
 
 namespace geon {
 
@@ -52,10 +53,9 @@ struct CameraDesc {
 };
 
 enum : int { MIXED_REPROJECT = 1, MIXED_ORBIT = 2, MIXED_NULLFIX = 4 };
-// mixed-kernel variants: register cap (none, 64, 51 registers) x block size
-// (128, 64, 256; block sizes other than 128 only for the equatorial source)
+// mixed-kernel variants of camera rays and ray arrays: register cap (none, 64,
+// 51 registers); of the equatorial source: sweep_rule.h
 constexpr int MIXED_CAPS = 3;
-constexpr int MIXED_VARIANTS = 9;
 
 // A regular grid of points for curvature jobs (geon_grid of the ABI).
 struct GridDesc {
@@ -124,7 +124,8 @@ struct TraceLaunch {
   // mixed precision
   float band;          // FP64 band half-width in the metric's own scale (0 = no band)
   float reserve_per_sm;  // persistent grid leaves this many blocks per SM free (may be fractional)
-  int variant;         // mixed kernel register-cap variant (0: none, 1: 8 blocks/SM, 2: 10)
+  int variant;         // mixed kernel register-cap variant (0: none, 1: 8 blocks/SM, 2: 10); of an
+                       // equatorial source also its block size, or SWEEP_BY_SIZE
   int mixed_flags;     // MIXED_* bits
   int decide;          // shadow rays whose class is all a caller needs (bisection rounds): the mixed
                        // path ends a ray as soon as its class is settled (MixedCore::decided_k)

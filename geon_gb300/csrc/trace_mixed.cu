@@ -867,15 +867,14 @@ static cudaError_t launch_mst_v(const TraceLaunch& L, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Rays that give every SM quarter `warps` warps.
-static int64_t rays_for(int warps) {
+static int device_sms() {
   static int sms = 0;
   if (sms == 0) {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  return (int64_t)sms * 4 * 32 * warps;
+  return sms;
 }
 
 template <int K, int SRC, int SINK>
@@ -901,13 +900,10 @@ static cudaError_t launch_mst(const TraceLaunch& L, cudaStream_t s) {
   }
   if constexpr (SRC == SRC_EQUATORIAL && SINK == SINK_SHADOW) {
     if (L.decide) return launch_mst_v<K, SRC, SINK, 1, FEAT_DECIDE | FEAT_CHAIN>(L, s);  // bisection rounds
-    // one warp per SM quarter: the chain of a step sets the time (19000 rays 17.0
-    // against 17.3 ms; from two warps on the combined test is the faster one:
-    // 38000 rays 21.9 against 22.9 ms)
-    if (L.n <= rays_for(1)) return launch_mst_v<K, SRC, SINK, 1, FEAT_CHAIN>(L, s);
-    // variant = register cap + 3 * block size (128, 64, 256); the same caps in
-    // registers per thread (64, 51) at every block size
-    switch (L.variant) {
+    // (FEAT_CHAIN and one-warp blocks: sweep_kernel says where and why)
+    switch (sweep_kernel(L.variant, L.n, device_sms(), L.started != nullptr)) {
+      case SWEEP_CHAIN: return launch_mst_v<K, SRC, SINK, 1, FEAT_CHAIN>(L, s);
+      case SWEEP_RESIDENT: return launch_mst_v<K, SRC, SINK, 1, 0, 32>(L, s);
       case 1: return launch_mst_v<K, SRC, SINK, 8, 0>(L, s);
       case 2: return launch_mst_v<K, SRC, SINK, 10, 0>(L, s);
       case 3: return launch_mst_v<K, SRC, SINK, 1, 0, 64>(L, s);
@@ -916,16 +912,8 @@ static cudaError_t launch_mst(const TraceLaunch& L, cudaStream_t s) {
       case 6: return launch_mst_v<K, SRC, SINK, 1, 0, 256>(L, s);
       case 7: return launch_mst_v<K, SRC, SINK, 4, 0, 256>(L, s);
       case 8: return launch_mst_v<K, SRC, SINK, 5, 0, 256>(L, s);
-      default: break;
+      default: return launch_mst_v<K, SRC, SINK, 1, 0>(L, s);
     }
-    // the GPU holds every ray at once (32 one-warp blocks per SM): dealt by quarter
-    // (60000 / 80000 / 120000 rays 38.6 / 38.8 / 39.7 -> 20.5 / 28.4 / 37.3 ms)
-    if (L.started) return launch_mst_v<K, SRC, SINK, 1, 0, 32>(L, s);
-    // more rays: the queue, with blocks of 64 threads, or of 128 at 51 registers
-    // and a tenth block per SM once the rays are over twice the lanes (300000
-    // rays 82 against 90 ms, 2^20 rays 275 against 272)
-    if (L.n > rays_for(18)) return launch_mst_v<K, SRC, SINK, 10, 0>(L, s);
-    return launch_mst_v<K, SRC, SINK, 1, 0, 64>(L, s);
   } else {
     // Minkowski's step is a few additions: its constants stay in registers
     // (16 x 16 pixels 1.10 against 1.17 ms, 256 x 256 2.64 against 2.68)

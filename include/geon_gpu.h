@@ -279,18 +279,26 @@ void geon_set_persistent_reserve_f(double blocks_per_sm);
 /* Launch variant of the mixed kernel per metric kind and ray source (source 0:
  * camera rays and ray arrays, 1: equatorial shadow rays). Register cap c: 0 =
  * none, 1 = at most 64 registers per thread, 2 = at most 51. Source 0 takes
- * variant = c (blocks of 128 threads); source 1 takes variant = c + 3 b with
- * block size b: 0 = 128, 1 = 64, 2 = 256 threads (source 1,
- * variant 0: the cap that suits the number of rays). geon_autotune_mixed times
- * every variant on calibration jobs of this metric (n_rays rays - 0 picks four
- * per lane of the widest grid - at most max_steps each; the equatorial job only
- * for Schwarzschild), selects the fastest per source and writes ray-steps/s to
- * rates_out[12] (3 for source 0, then 9 for source 1) and the choices to
- * best_out[2] (-1 = source not tuned); either may be NULL. The persistent
- * reserve (geon_set_persistent_reserve) counts slots of 128 threads whatever
- * the block size. */
+ * variant = c (blocks of 128 threads; default 0); source 1 takes variant =
+ * c + 3 b with block size b: 0 = 128, 1 = 64, 2 = 256 threads, at every number of
+ * rays, or 9, the default: the kernel that suits the number of rays (some of them
+ * are none of the nine). geon_set_sweep_variant_above sets a variant of source 1
+ * for classifications of more than `rays` rays only, smaller ones running as with
+ * 9 (rays 0: geon_set_mixed_variant); geon_get_sweep_variant_above tells that
+ * number. geon_autotune_mixed times every variant on calibration jobs of this
+ * metric (n_rays rays - 0 picks four per lane of the widest grid - at most
+ * max_steps each; the equatorial job only for Schwarzschild) and writes
+ * ray-steps/s to rates_out[12] (3 for source 0, then 9 for source 1) and the
+ * choices to best_out[2] (-1 = source not tuned); either may be NULL. It selects
+ * the fastest for source 0. Source 1 keeps 9 unless the calibration has more rays
+ * than the GPU holds at once (1024 per SM) and a variant is over 2 % faster there
+ * than the kernel of 9; it is then set above that many rays. The persistent
+ * reserve (geon_set_persistent_reserve) counts slots of 128 threads whatever the
+ * block size. */
 int geon_set_mixed_variant(int kind, int source, int variant);
 int geon_get_mixed_variant(int kind, int source);
+int geon_set_sweep_variant_above(int kind, int variant, int64_t rays);
+int64_t geon_get_sweep_variant_above(int kind);
 int geon_autotune_mixed(geon_metric_t m, int64_t n_rays, int64_t max_steps, double* rates_out,
                         int* best_out);
 
