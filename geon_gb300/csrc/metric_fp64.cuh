@@ -609,6 +609,23 @@ __device__ __forceinline__ bool rk4_step(const MetricDesc& M, const double y[8],
   return ok;
 }
 
+// What the state before a step tells about rk4_step_schw_soft: false where it
+// would fail (some of what it tests at the end).
+__device__ __forceinline__ bool soft_step_starts(const MetricDesc& M, const double y[8], double half_h, double sixth) {
+  uint32_t worst = sf::spread(M.p[0]);
+  const uint32_t ds = sf::spread(sixth), dh = sf::spread(half_h);
+  worst = ds > worst ? ds : worst;
+  worst = dh > worst ? dh : worst;
+#pragma unroll
+  for (int i = 4; i < 8; ++i) {
+    const uint32_t d = sf::spread(y[i]);
+    worst = d > worst ? d : worst;
+  }
+  double k;
+  int q;
+  return dm::quadrant_by_word(y[2], k, q) && worst < sf::RANGE;
+}
+
 // rk4_step of Schwarzschild with its multiplications in the integer pipes:
 // about 220 of the step's 390 FP64 operations stay on the FP64 pipe, which both
 // kinds of pipe then share evenly. The same bits; false (out not written) when an

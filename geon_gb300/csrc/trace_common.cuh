@@ -161,6 +161,7 @@ __device__ __forceinline__ int64_t group_steps(Stepper& st, const TraceLaunch& L
   const int left = left64 < (int64_t)TRACE_INNER ? (int)left64 : TRACE_INNER;
   int done = 0, extra = 0;
   t = TERM_NONE;
+  st.group_begin(L);
 #pragma unroll 1
   for (; done < left; ++done) {
     if constexpr (Stepper::FAST) {  // steps the stepper can take with fewer tests
@@ -188,7 +189,8 @@ __device__ __forceinline__ int64_t group_steps(Stepper& st, const TraceLaunch& L
 }
 
 // geodesic.rs:62-117 for every ray of the job, persistent over a work queue.
-// Stepper owns the ray state: load(y0), to_double(y), terminate(L), step(L)
+// Stepper owns the ray state: load(y0), to_double(y), group_begin(L) and
+// group_end(L) around the steps between two refills, terminate(L), step(L)
 // returning STEP_OK (advanced), STEP_NONFINITE (state unchanged: Diverged) or
 // STEP_HORIZON (state unchanged: Captured after this step). Where Stepper::FAST,
 // fast_steps(L, left) takes some of the next `left` steps (their termination tests

@@ -761,6 +761,7 @@ struct MixedStepper : MixedCore<FEAT> {
   __device__ __forceinline__ int fast_steps(const TraceLaunch& L, int left) {
     return this->template fast_steps_k<K>(L, left);
   }
+  __device__ __forceinline__ void group_begin(const TraceLaunch&) {}
   __device__ __forceinline__ void group_end(const TraceLaunch& L) { this->template group_end_k<K>(L); }
   __device__ __forceinline__ void check_null(const TraceLaunch& L, const double y0[8]) {
     this->template check_null_k<K>(L, y0);
@@ -818,6 +819,7 @@ struct MixedStepperAny : MixedCore<FEAT> {
   __device__ __forceinline__ int fast_steps(const TraceLaunch& L, int left) {
     return on_kind([&](auto k) { return this->template fast_steps_k<decltype(k)::value>(L, left); });
   }
+  __device__ __forceinline__ void group_begin(const TraceLaunch&) {}
   __device__ __forceinline__ void group_end(const TraceLaunch& L) {
     on_kind([&](auto k) { this->template group_end_k<decltype(k)::value>(L); });
   }
