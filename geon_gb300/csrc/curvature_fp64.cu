@@ -825,17 +825,6 @@ constexpr bool has_point_kernel() {
   return K == KIND_ALCUBIERRE || K == KIND_MORRIS_THORNE || K == KIND_SCHWARZSCHILD;
 }
 
-// The point kernel from this many points on. Below, the SMs are not full with
-// one thread per point and the time is one thread's chain of operations (254 us
-// for an Alcubierre grid point with 16 vectors, 91 and 87 us for Morris-Thorne
-// and Schwarzschild, whatever the number of points up to ~16384), while the
-// cooperative kernel's grows with the points: it takes 99 / 202 us for 3840 /
-// 8192 Alcubierre points, 59 / 81 us for 2048 / 4096 Morris-Thorne points.
-template <int K>
-constexpr int64_t point_min() {
-  return K == KIND_ALCUBIERRE ? 9216 : 5120;
-}
-
 template <int K, bool GRID>
 static cudaError_t launch_point_k(const MetricDesc& M, int what, const double* x, int64_t n, const double* k,
                                   int64_t nk, int k_shared, double* out, int* flags, const GridDesc& grid,
@@ -859,7 +848,7 @@ static cudaError_t launch_curv_k(const MetricDesc& M, int what, const double* x,
                                  int64_t nk, int k_shared, double* out, int* flags, const GridDesc& grid,
                                  uint64_t seed, double* out2, double* kout, cudaStream_t s) {
   if constexpr (has_point_kernel<K>()) {
-    if (what != 0 && n >= point_min<K>())
+    if (what != 0 && one_thread_per_point(K == KIND_ALCUBIERRE, GRID, n, what >= 5 ? nk : 0, device_sms()))
       return launch_point_k<K, GRID>(M, what, x, n, k, nk, k_shared, out, flags, grid, seed, out2, kout, s);
   }
   const size_t smem = curv_smem_doubles<K>() * sizeof(double);

@@ -6,6 +6,7 @@
 #include <string>
 
 #include "../../include/geon_gpu.h"
+#include "curvature_rule.h"
 #include "sweep_rule.h"
 
 namespace geon {
@@ -142,6 +143,17 @@ struct TraceLaunch {
   unsigned quarters;
   int* flags;                 // bit 0: a metric became singular (inverse of g failed)
 };
+
+// SMs of the device (queried once).
+inline int device_sms() {
+  static const int sms = [] {
+    int dev = 0, count = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+    return count;
+  }();
+  return sms;
+}
 
 // ---- launchers (trace_fp64.cu) ----
 cudaError_t launch_trace_fp64(const TraceLaunch& L, int src, int sink, cudaStream_t s);

@@ -869,16 +869,6 @@ static cudaError_t launch_mst_v(const TraceLaunch& L, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-static int device_sms() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return sms;
-}
-
 template <int K, int SRC, int SINK>
 static cudaError_t launch_mst(const TraceLaunch& L, cudaStream_t s) {
   const int feat = ((K != KIND_MINKOWSKI && L.band > 0.0f) ? FEAT_BAND : 0) |
