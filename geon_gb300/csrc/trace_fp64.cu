@@ -460,11 +460,11 @@ __global__ void pointwise_kernel(const MetricDesc M, int what, const double* __r
 //   wormhole Gamma    33 -> 33    50 -> 46    86 -> 84   190 -> 201
 //   sampled Gamma    500 -> 119  570 -> 132  612 -> 465 1200 -> 1720
 // 8 lanes take up to 8 times the FP64 work of a thread's chain, so they win while
-// the chip has quarters to spare: up to FEW_POINTS, 16 warps per SM, for every
+// the chip has quarters to spare: up to FEW_POINTS_PER_SM, 16 warps, for every
 // metric (at 19456 the sampled metric already loses, 640 -> 888).
 // ---------------------------------------------------------------------------
 constexpr int FEW_LANES = 8;
-constexpr int64_t FEW_POINTS = 152 * 64;
+constexpr int64_t FEW_POINTS_PER_SM = 64;
 
 __device__ __forceinline__ double of_lane(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane, FEW_LANES); }
 
@@ -564,7 +564,7 @@ cudaError_t launch_pointwise(const MetricDesc& M, int what, const double* in, in
   if (n <= 0) return cudaSuccess;
   const int block = 128;
   const unsigned grid = (unsigned)((n + block - 1) / block);
-  if (n <= FEW_POINTS && few_differences(M.kind, what)) {
+  if (n <= FEW_POINTS_PER_SM * device_sms() && few_differences(M.kind, what)) {
     const unsigned few = (unsigned)((n + 32 / FEW_LANES - 1) / (32 / FEW_LANES));
     switch (M.kind) {
       case KIND_SCHWARZSCHILD: few_points_kernel<KIND_SCHWARZSCHILD><<<few, 32, 0, s>>>(M, what, in, n, out, flags); break;
