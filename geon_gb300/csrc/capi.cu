@@ -29,7 +29,7 @@ thread_local std::string g_last_error;
 std::atomic<int> g_show_stars{1};
 // Mixed-precision options: FP64 band half-width per metric kind (in units of
 // M, b0, s; 0 disables) and the null re-projection switch.
-std::atomic<float> g_band[4] = {{0.0f}, {0.0f}, {0.0f}, {0.0f}};
+std::atomic<float> g_band[KIND_FIELD + 1] = {};  // (a sampled metric has none: 0)
 std::atomic<int> g_reproject{0};
 std::atomic<int> g_orbit{1};  // orbit-plane frame of the mixed path (default on)
 std::atomic<int> g_nullfix{1};  // compensated null re-projection every 16 steps (planar steps; default on)
@@ -39,8 +39,9 @@ std::atomic<double> g_rtol{1e-10};  // GEON_ADAPTIVE error tolerances
 std::atomic<double> g_atol{1e-12};
 // Mixed-kernel variant per metric kind of camera rays and ray arrays, and of
 // equatorial rays (sweep_choice), set by the caller or by geon_autotune_mixed.
-std::atomic<int> g_variant[4] = {{0}, {0}, {0}, {0}};
-std::atomic<int64_t> g_sweep[4] = {{SWEEP_BY_SIZE}, {SWEEP_BY_SIZE}, {SWEEP_BY_SIZE}, {SWEEP_BY_SIZE}};
+std::atomic<int> g_variant[KIND_FIELD + 1] = {};
+std::atomic<int64_t> g_sweep[KIND_FIELD + 1] = {{SWEEP_BY_SIZE}, {SWEEP_BY_SIZE}, {SWEEP_BY_SIZE}, {SWEEP_BY_SIZE},
+                                                {SWEEP_BY_SIZE}};
 // Kernels launched by this library since load (ours only; memsets excluded).
 std::atomic<unsigned long long> g_launches{0};
 inline void counted(unsigned long long n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
@@ -221,6 +222,9 @@ MixedConsts mixed_consts(const MetricDesc& M, double step, double half_step, dou
 }
 
 TraceLaunch base_launch(geon_metric_t m, double step, int64_t max_steps) {
+  // every kind of metric comes here, the sampled one too
+  static_assert(sizeof g_band / sizeof *g_band > KIND_FIELD && sizeof g_variant / sizeof *g_variant > KIND_FIELD &&
+                sizeof g_sweep / sizeof *g_sweep > KIND_FIELD, "options of every kind of metric");
   TraceLaunch L;
   std::memset(&L, 0, sizeof L);
   L.M = m->desc;
