@@ -562,11 +562,13 @@ struct MixedCore {
   // touched). The arithmetic is step_fp32_planar_k's with the factor -2 of the
   // p^t and p^phi derivatives moved into the constants they meet (scaling by a
   // power of two is exact), which saves a multiplication per right-hand side;
-  // the same bits.
+  // the same bits for momenta that keep the derivatives clear of FP32's ends,
+  // where a product and its double round or overflow apart (ordinary_momenta).
   template <int K>
   __device__ __forceinline__ int planar_steps_k(const MixedConsts& Q, int left) {
     constexpr bool S = K == KIND_SCHWARZSCHILD;
     constexpr bool TIME = (FEAT & FEAT_NO_TIME) == 0;
+    if (!ordinary_momenta()) return 0;
     if (!S && !TIME) fast_two_sum_update(hi[4], lo[4], 0.0f);  // p^t: a zero increment each step
     int done = 0;
 #pragma unroll 1
@@ -615,6 +617,13 @@ struct MixedCore {
       count_step();
     }
     return done;
+  }
+  // Momenta at the start of a group for which planar_steps_k has the bits of
+  // step_fp32_planar_k: below 2^45, p^t from 2^-40 up, p^phi from there or zero. (A p^r
+  // that is smaller for a stage or two does not show: its terms meet larger ones.)
+  __device__ __forceinline__ bool ordinary_momenta() const {
+    const float p0 = fabsf(hi[4]), p3 = fabsf(hi[7]);
+    return (max_nan(p0, fabsf(hi[5]), p3) < 0x1p45f) & (p0 >= 0x1p-40f) & ((p3 >= 0x1p-40f) | (p3 == 0.0f));
   }
   // the largest of three, NaN if one is NaN
   static __device__ __forceinline__ float max_nan(float a, float b, float c) {
@@ -828,6 +837,7 @@ struct MixedStepperAny : MixedCore<FEAT> {
   }
 };
 
+#ifndef GEON_STEPPERS_ONLY  // (a test compiles the steppers alone)
 // MINB is the register cap chosen by the autotuner: __launch_bounds__(BLOCK,
 // MINB) asks the compiler to fit MINB blocks per SM (1: no cap, 56 registers
 // and 9 blocks of 128 for the planar equatorial step, 59 and 8 for the camera
@@ -1112,5 +1122,7 @@ cudaError_t launch_trace_mixed(const TraceLaunch& L, int src, int sink, cudaStre
   }
   return cudaErrorInvalidValue;
 }
+
+#endif  // GEON_STEPPERS_ONLY
 
 }  // namespace geon
