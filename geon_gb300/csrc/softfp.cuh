@@ -107,9 +107,12 @@ GEON_SF double unit53(uint64_t v) {
   return from_words((uint32_t)(m >> 32) + ((uint32_t)(1032 - z) << 20), (uint32_t)m);
 }
 
-// Estimates of 1/x (x in [1, 2]) and 1/sqrt(x) (x in [1, 4]) as FP32 bits,
-// relative error at most 2^-23 and 2^-22.4 (PTX rcp.approx, rsqrt.approx). On
-// the host `est_error` moves them by units in the last place (tests).
+// Estimates of 1/x (x in [1, 2]) and 1/sqrt(x) (x in [1, 4]) as FP32 bits (PTX
+// rcp.approx, rsqrt.approx). What follows holds for relative errors up to RCP_ERROR
+// (2^-22) and RSQRT_ERROR (2^-22.4); the hardware's are 2^-23.28 and 2^-22.94 at
+// most, which a test measures over all these arguments. On the host the tests move
+// the estimates, by units in the last place or by a part of those errors.
+constexpr double RCP_ERROR = 0x1p-22, RSQRT_ERROR = 0x1.8p-23;
 #ifdef __CUDA_ARCH__
 GEON_SF uint32_t rcp_bits(uint32_t x) {
   float r;
@@ -128,21 +131,29 @@ inline int& est_error() {
   static int e = 0;
   return e;
 }
-inline uint32_t rcp_bits(uint32_t x) {
-  float f, r;
-  memcpy(&f, &x, 4);
-  r = (float)(1.0 / (double)f);
+inline double& est_relative() {  // as a part of the bound, -1 to 1
+  static double e = 0.0;
+  return e;
+}
+// the FP32 number next to v (1 + e) on v's side (e = 0: nearest to v), moved by units
+inline uint32_t moved(double v, double e) {
+  const double w = v * (1.0 + e);
+  float r = (float)w;
+  if (e > 0.0 && (double)r > w) r = nextafterf(r, 0.0f);
+  if (e < 0.0 && (double)r < w) r = nextafterf(r, 2.0f);
   uint32_t u;
   memcpy(&u, &r, 4);
   return u + est_error();
 }
-inline uint32_t rsqrt_bits(uint32_t x) {
-  float f, r;
+inline uint32_t rcp_bits(uint32_t x) {
+  float f;
   memcpy(&f, &x, 4);
-  r = (float)(1.0 / sqrt((double)f));
-  uint32_t u;
-  memcpy(&u, &r, 4);
-  return u + est_error();
+  return moved(1.0 / (double)f, RCP_ERROR * est_relative());
+}
+inline uint32_t rsqrt_bits(uint32_t x) {
+  float f;
+  memcpy(&f, &x, 4);
+  return moved(1.0 / sqrt((double)f), RSQRT_ERROR * est_relative());
 }
 inline uint32_t umulhi(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
 inline int32_t smulhi(int32_t a, int32_t b) { return (int32_t)(((int64_t)a * b) >> 32); }
@@ -171,10 +182,11 @@ GEON_SF uint32_t fixed31(uint32_t r) {
 
 // Significand (53 bits) of a / b rounded to nearest, for significands A' in
 // [B, 2B) and B in [2^52, 2^53). Y = 2^31 times an estimate of 2^52 / B with
-// relative error e at most 2^-21.7 (two units in the last place of the
-// estimate, 2^-22, and its argument's 2^-24; the hardware's is one unit).
-//   d1 ~ (A'/B) 2^30 < 2^31: error < 2^9.3 + 2  =>  |R1| < 2^9.4 B < 2^62.4
-//   d2 ~ R1/B 2^19, |d2| < 2^28.4: error < 2^6.7 + 2  =>  |R2| < 2^6.8 B
+// relative error e at most 2^-21.67 (the estimate's RCP_ERROR = 2^-22 and its
+// argument's 2^-24; the clamp moves a value beyond an end of [1/2, 1) to the end or,
+// for B = 2^52, from 1 by 2^-24).
+//   d1 ~ (A'/B) 2^30 < 2^31: error < 2^9.33 + 2  =>  |R1| < 2^9.4 B < 2^62.4
+//   d2 ~ R1/B 2^19, |d2| < 2^28.4: error < 2^6.73 + 2  =>  |R2| < 2^6.8 B
 //   d3 ~ floor(R2/B 2^3): error in [0, 1] and a part in 2^11 either way, so the
 // quotient is Q = d1 2^22 + d2 2^3 + d3 plus R3 / B with R3 in (-B/2^11, 1.01 B).
 GEON_SF uint64_t quotient(uint64_t A, uint64_t B, uint32_t Y) {
@@ -235,8 +247,9 @@ GEON_SF double rcp(double b) { return outside(hi_of(b)) ? 1.0 / b : rcp_inside(b
 
 // sqrt(a), rounded to nearest: the bits of the IEEE square root. With n in
 // [1, 4) the significand (times 2 for an odd exponent), A = n 2^52, and y the
-// estimate of 1/sqrt(n) (relative error at most 2^-22.9, argument 2^-24, clamp
-// 2^-24: together 2^-22), Y = 2^31 y:
+// estimate of 1/sqrt(n) (relative error at most RSQRT_ERROR = 2^-22.4, and half its
+// argument's 2^-23: together 2^-22; the clamp only brings a value nearer, or moves
+// 1 by 2^-24), Y = 2^31 y:
 //   S1 ~ sqrt(n) 2^30: error < 2^9.1, R1 = n 2^60 - S1^2, |R1| < 2^41.1
 //   d2 ~ R1 y 2^-12 (half the remainder over the root, 2^19 times finer):
 //     T = S1 2^19 + d2 ~ sqrt(n) 2^49: error < 2^7.3, R2 = n 2^98 - T^2, |R2| < 2^58.3
