@@ -690,9 +690,12 @@ __device__ __forceinline__ SparseTetrad sparse_tetrad(const double* g) {
   return t;
 }
 
-// what: as curvature_kernel, 1 to 6.
+// what: as curvature_kernel, 1 to 6. Blocks per SM: as many as the registers of the
+// sparse path let in; the dense functions, which hardly a point calls, would set
+// them for the whole kernel (156-166 registers and 6 blocks per SM: R at 60000 points
+// 872 us for Alcubierre, 142 for Morris-Thorne, whole calls; 753 and 131 as it is).
 template <int K, bool GRID>
-__global__ void __launch_bounds__(POINT_THREADS)
+__global__ void __launch_bounds__(POINT_THREADS, K == KIND_SCHWARZSCHILD ? 12 : 10)
 curvature_point_kernel(const MetricDesc M, int what, const double* __restrict__ xs, int64_t n,
                        const double* __restrict__ ks, int64_t nk, int k_shared, double* __restrict__ out, int* flags,
                        const GridDesc grid, uint64_t seed, double* __restrict__ out2, double* __restrict__ kout) {
