@@ -21,14 +21,14 @@ namespace geon {
 //    threads (0.26 ns a point and vector): Morris-Thorne 5120 points with 16 / 64 / 256
 //    vectors 93 / 109, 270 / 200, 982 / 568; 9728 with 64 / 256 271 / 261, 981 / 753;
 //    14592 with 256 / 1024 1120 / 1124, 4371 / 4078; 19456 with 256 1120 / 1497. The
-//    crossing lies at nk (112 - points per SM) = 1850, and for Alcubierre grids at
+//    crossing lies at nk (112 - points per SM) = 2100, and for Alcubierre grids at
 //    1100 (14592 points: nk = 87).
 inline bool one_thread_per_point(bool alcubierre, bool grid, int64_t n, int64_t nk, int sms) {
   const int64_t least = alcubierre ? (grid ? (int64_t)96 * sms + 1 : (int64_t)128 * sms + 1) : (int64_t)33 * sms;
   if (n < least) return false;
   const int64_t free = (int64_t)112 * sms - n;
   if (free <= 0 || nk <= 0) return true;
-  return nk <= (alcubierre ? 1100 : 1850) * (int64_t)sms / free;
+  return nk <= (alcubierre ? 1100 : 2100) * (int64_t)sms / free;
 }
 
 }  // namespace geon
