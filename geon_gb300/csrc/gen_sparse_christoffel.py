@@ -418,7 +418,8 @@ def build(name, doc, spec, depends_on, evaluator):
            "double k[8]) {",
            "  const double* x = y;",
            "  bool singular;"]
-    rhs += gen.lines[:n0] + sums
+    # (a right-hand side calls one copy of the metric evaluation where there is one)
+    rhs += [line.replace("alc_g00_g01(", "alc_g00_g01_called(") for line in gen.lines[:n0]] + sums
     rhs += ["  k[0] = y[4]; k[1] = y[5]; k[2] = y[6]; k[3] = y[7];"] + rl
     rhs += ["  return !singular;", "}"]
     return "\n".join(out) + "\n\n" + "\n".join(frm) + "\n\n" + "\n".join(rhs), gen

@@ -88,16 +88,38 @@ __device__ __forceinline__ bool inv4(const double a[16], double out[16]) {
 // finite-difference fallback. metric_g and the sparse Christoffel code both
 // call these, so both see the same bits.
 // ---------------------------------------------------------------------------
+// f(r_s) of alcubierre.rs:33-47
+__device__ __forceinline__ double alc_shape(double r_s, double R, double s, double denom) {
+  const double t_plus = dm::tanh_det(sf::div(r_s + R, s));
+  const double t_minus = dm::tanh_det(sf::div(r_s - R, s));
+  return sf::div(t_plus - t_minus, denom);
+}
+// One copy of it per kernel, for the right-hand sides, which evaluate it 7 times:
+// inlined (14 tanh with their integer divisions) the step outgrew the instruction
+// cache once the warps of an SM were at different points of it. 30000 FP64 rays
+// around a bubble with s = 0.5, 400 steps: 221 ms inlined, 97 called (199 inlined with
+// divisions on the FP64 pipe); 2000 rays 80 and 61 (106); 100 adaptive steps of 30000
+// rays 119 and 66. Point and curvature kernels, a few copies each, lose by the call
+// (R at 4000 points 106 and 115 us).
+static __device__ __noinline__ double alc_shape_called(double r_s, double R, double s, double denom) {
+  return alc_shape(r_s, R, s, denom);
+}
+
 // alcubierre.rs:33-63: g_tt = -1 + v^2 f^2, g_tx = g_xt = -v f
-__device__ __forceinline__ void alc_g00_g01(const MetricDesc& M, const double x[4], double* g00, double* g01) {
+template <bool CALL>
+__device__ __forceinline__ void alc_g00_g01_by(const MetricDesc& M, const double x[4], double* g00, double* g01) {
   const double R = M.p[0], s = M.p[1], v = M.p[2], ship_x = M.p[3];
   const double dx = x[1] - ship_x, dy = x[2], dz = x[3];
   const double r_s = sf::root(dx * dx + dy * dy + dz * dz);
-  const double t_plus = dm::tanh_det(sf::div(r_s + R, s));
-  const double t_minus = dm::tanh_det(sf::div(r_s - R, s));
-  const double f = sf::div(t_plus - t_minus, M.alc_denom);
+  const double f = CALL ? alc_shape_called(r_s, R, s, M.alc_denom) : alc_shape(r_s, R, s, M.alc_denom);
   *g00 = -1.0 + v * v * f * f;
   *g01 = -v * f;
+}
+__device__ __forceinline__ void alc_g00_g01(const MetricDesc& M, const double x[4], double* g00, double* g01) {
+  alc_g00_g01_by<false>(M, x, g00, g01);
+}
+__device__ __forceinline__ void alc_g00_g01_called(const MetricDesc& M, const double x[4], double* g00, double* g01) {
+  alc_g00_g01_by<true>(M, x, g00, g01);
 }
 
 // morris_thorne.rs:22-36: g_thth = b0^2 + l^2, g_phph = (b0^2 + l^2) sin^2(theta)
