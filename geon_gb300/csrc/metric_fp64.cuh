@@ -589,7 +589,8 @@ __device__ __forceinline__ bool geodesic_rhs(const MetricDesc& M, const double y
 // Classical RK4 (integrator.rs:16-40) with the reference's grouping:
 // y + (0.5*h)*k, y + h*k3, and y + (h/6)*(((k1 + 2 k2) + 2 k3) + k4). The
 // stages run in a loop: the right-hand side is a thousand instructions and more,
-// and one copy of it stays in the instruction cache. k1 + 2 k2 is one fused
+// and one copy of it stays in the instruction cache (Minkowski's is four moves: one ray
+// of 400 steps 776 us in a loop, 623 unrolled). k1 + 2 k2 is one fused
 // operation with the same bits, since 2 k2 is exact; only where 2 k2 or 2 k3
 // overflows (or is not a number) could the two differ, and there the
 // reference's sum is infinite or NaN, so *finite reports it with the
@@ -602,7 +603,7 @@ __device__ __forceinline__ bool rk4_step(const MetricDesc& M, const double y[8],
 #pragma unroll
   for (int i = 0; i < 8; ++i) ys[i] = y[i];
   bool ok = true;
-#pragma unroll 1
+#pragma unroll (K == KIND_MINKOWSKI ? 3 : 1)
   for (int stage = 0; stage < 3; ++stage) {
     ok &= geodesic_rhs<K>(M, ys, k);
     const double c = stage < 2 ? half_h : h;
