@@ -190,19 +190,23 @@ int make_camera(geon_metric_t m, const geon_camera* cam, int64_t spa, CameraDesc
   return GEON_OK;
 }
 
+BandConsts band_consts(const MetricDesc& M) {
+  const double dn = M.kind == GEON_ALCUBIERRE ? M.alc_denom : 1.0;  // 2 tanh(R/s)
+  return {1.0 / M.p[1], 1.0 / dn, 1.0 / (dn * M.p[1])};
+}
+
 // The mixed path's FP32 constants: each the FP64 value rounded once.
-MixedConsts mixed_consts(const MetricDesc& M, double step, double half_step, double sixth, int64_t max_steps) {
+MixedConsts mixed_consts(const MetricDesc& M, const BandConsts& b, double step, double half_step, double sixth, int64_t max_steps) {
   MixedConsts c;
   c.m = (float)M.p[0];
   c.two_m = (float)(2.0 * M.p[0]);
   c.b0sq = (float)(M.p[0] * M.p[0]);
   c.R = (float)M.p[0];
-  c.inv_s = (float)(1.0 / M.p[1]);
+  c.inv_s = (float)b.inv_s;
   c.v = (float)M.p[2];
   c.ship_x = (float)M.p[3];
-  const double dn = M.kind == GEON_ALCUBIERRE ? M.alc_denom : 1.0;  // 2 tanh(R/s)
-  c.fnorm = (float)(1.0 / dn);
-  c.dfnorm = (float)(1.0 / (dn * M.p[1]));
+  c.fnorm = (float)b.fnorm;
+  c.dfnorm = (float)b.dfnorm;
   c.cap_hi = (float)M.capture_r;
   c.cap_lo = (float)(M.capture_r - (double)c.cap_hi);
   c.esc_hi = (float)M.escape_r;
@@ -232,7 +236,8 @@ TraceLaunch base_launch(geon_metric_t m, double step, int64_t max_steps) {
   L.half_step = 0.5 * step;
   L.sixth = step / 6.0;
   L.max_steps = max_steps;
-  L.mx = mixed_consts(L.M, L.step, L.half_step, L.sixth, max_steps);
+  L.bc = band_consts(L.M);
+  L.mx = mixed_consts(L.M, L.bc, L.step, L.half_step, L.sixth, max_steps);
   L.band = g_band[m->desc.kind].load();
   L.mixed_flags = (g_reproject.load() ? MIXED_REPROJECT : 0) | (g_orbit.load() ? MIXED_ORBIT : 0) |
                   (g_nullfix.load() ? MIXED_NULLFIX : 0);

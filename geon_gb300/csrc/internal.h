@@ -94,11 +94,17 @@ struct MixedConsts {
   float cap_steps;                               // the step cap, for the early decision's budget test
 };
 
+// Alcubierre's constants of the FP64 band steps: 1/s, 1/(2 tanh(R/s)) and that over s.
+struct BandConsts {
+  double inv_s, fnorm, dfnorm;
+};
+
 constexpr unsigned RESIDENT_QUARTERS = 4096;  // more than 4 per SM of any device
 
 struct TraceLaunch {
   MetricDesc M;
   MixedConsts mx;
+  BandConsts bc;
   CameraDesc cam;
   int64_t n;           // rays in the job
   double step;

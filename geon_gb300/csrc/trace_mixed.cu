@@ -680,7 +680,7 @@ struct MixedCore {
   template <int K>
   __device__ __forceinline__ int step_fp64_k(const TraceLaunch& L) {
     AConsts<double> Cd;
-    Cd.init(L.M);
+    Cd.init(L.M, L.bc);
     double y[8];
     to_double_k<K>(y);
     double s0 = 0.0, c0 = 1.0;
