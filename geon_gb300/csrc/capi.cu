@@ -1082,12 +1082,8 @@ int geon_equatorial_rays(geon_metric_t m, double r_obs, const double* alpha, siz
 }
 
 // Classify rays launched at the given angles on stream s (device buffers).
-// Sweeps of at least SHADOW_ORDER_MIN rays (and fewer than 2^31) are claimed
-// longest first (launch_shadow_order); smaller ones, two warps per SM quarter and
-// less, in index order: they take as long as one ray does either way (60000 rays
-// 28.3 ms in order, 36.5 unordered; 38000 rays 20.7).
-constexpr int64_t SHADOW_ORDER_MIN = 40000;
-
+// Sweeps of more than two warps per SM quarter (sweep_ordered) are claimed longest
+// first (launch_shadow_order), smaller ones in index order.
 static int classify_dev(geon_metric_t m, double r_obs, const double* d_alpha, int64_t n, double step,
                         int64_t max_steps, int precision, int32_t* d_term, int64_t* d_steps,
                         cudaStream_t s) {
@@ -1105,7 +1101,7 @@ static int classify_dev(geon_metric_t m, double r_obs, const double* d_alpha, in
   GEON_CUDA(ws.alloc(ws_bytes, s));
   GEON_CUDA(cudaMemsetAsync(ws.p, 0, ws_bytes, s));
   const int32_t* order = nullptr;
-  if (g_sweep_order.load() && n >= SHADOW_ORDER_MIN && n < ((int64_t)1 << 31)) {
+  if (g_sweep_order.load() && sweep_ordered(n, sms)) {
     GEON_CUDA(dorder.alloc(sizeof(int32_t) * n, s));
     counted();
     GEON_CUDA(launch_shadow_order(m->desc.p[0], r_obs, d_alpha, n, dorder.as<int32_t>(),

@@ -28,16 +28,23 @@ inline int sweep_variant(int64_t choice, int64_t n) {
 inline int64_t sweep_one_warp(int sms) { return (int64_t)sms * 128; }
 inline int64_t sweep_held(int sms) { return (int64_t)sms * 1024; }
 
+// Claimed longest first? Up to two warps per SM quarter (256 rays per SM) a sweep
+// takes as long as its longest rays either way (20000 to 38900 rays 19.8 ms); from
+// the third warp on the order keeps the long rays apart (41000 / 60000 / 120000 rays
+// 20.0 / 20.3 / 36.8 ms in order, 27.6 / 36.0 / 60.6 not; 2^20 rays 269 and 290). The
+// order's indexes are 32-bit.
+inline bool sweep_ordered(int64_t n, int sms) { return n > 2 * sweep_one_warp(sms) && n < ((int64_t)1 << 31); }
+
 // The kernel of a sweep of n rays. `resident`: the launch has trace_resident's
 // workspace.
 //  - One warp per SM quarter: the chain of a step sets the time (19000 rays 17.0
 //    against 17.3 ms; from two warps on the combined test is the faster one:
 //    38000 rays 21.9 against 22.9 ms).
 //  - Everything held at once (32 one-warp blocks per SM): dealt by quarter (60000 /
-//    80000 / 120000 rays 38.6 / 38.8 / 39.7 -> 20.5 / 28.4 / 37.3 ms).
+//    120000 rays 20.3 / 36.8 ms; 28.9 / 46.2 from the queue, both longest first).
 //  - More rays: the queue, with blocks of 64 threads, or of 128 at 51 registers and
-//    a tenth block per SM once the rays are over twice the lanes (300000 rays 82
-//    against 90 ms, 2^20 rays 275 against 272).
+//    a tenth block per SM once the rays are over twice the lanes (300000 rays 80.7
+//    against 88.6 ms, 2^20 rays 270.2 against 267.3).
 inline int sweep_kernel(int variant, int64_t n, int sms, bool resident) {
   if (variant != SWEEP_BY_SIZE) return variant;
   if (n <= sweep_one_warp(sms)) return SWEEP_CHAIN;

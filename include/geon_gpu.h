@@ -363,7 +363,7 @@ int geon_shadow_bisect(geon_metric_t schwarzschild, double r_obs, const double* 
                        size_t nb, int iters, double step, int64_t max_steps, int precision,
                        double* alpha_c, double* lo_out, double* hi_out, int64_t* steps_out);
 
-/* Claim order of geon_shadow_classify(_dev) over 40000 rays or more: 1 (the
+/* Claim order of geon_shadow_classify(_dev) over more than 256 rays per SM: 1 (the
  * default) claims the rays whose impact parameter is at least 0.998 of the
  * critical one (escaping or orbiting near the photon sphere: the long paths)
  * first, so the short ones fill the end of the sweep when lanes run out of

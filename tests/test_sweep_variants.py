@@ -26,6 +26,7 @@ def rule(tmp_path_factory):
     lib.choice.restype, lib.choice.argtypes = ll, [i, ll]
     lib.chosen.argtypes = [ll, ll]
     lib.kernel.argtypes = [i, ll, i, i]
+    lib.ordered.argtypes = [ll, i]
     lib.tuned.restype, lib.tuned.argtypes = ll, [ctypes.POINTER(ctypes.c_double), ll, i]
     return lib
 
@@ -58,6 +59,12 @@ def test_tuned_choice(rule, n):
     assert tuned(better) == ((BY_SIZE,) * 3 if n <= HELD else (6, BY_SIZE, 6))
     better[queue] = 120.0
     assert tuned(better) == (BY_SIZE,) * 3
+
+
+@pytest.mark.parametrize("n,ordered", [(1, 0), (2 * ONE_WARP, 0), (2 * ONE_WARP + 1, 1), (39500, 1), (1 << 20, 1),
+                                       ((1 << 31) - 1, 1), (1 << 31, 0)])
+def test_claim_order_from_the_third_warp(rule, n, ordered):
+    assert rule.ordered(n, SMS) == ordered
 
 
 def test_setters_without_gpu():
@@ -113,7 +120,7 @@ def test_cached_choice(monkeypatch, tmp_path):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [700, ONE_WARP, 60001, HELD + 1, 18 * ONE_WARP + 1])
+@pytest.mark.parametrize("n", [700, ONE_WARP, 2 * ONE_WARP + 1, 60001, HELD + 1, 18 * ONE_WARP + 1])
 def test_every_variant_gives_the_same_results(geon, n):
     m = geon.Schwarzschild(1.0, 1.001, 30.0)
     alpha = np.radians(np.random.default_rng(n).uniform(10.0, 20.0, n))
