@@ -23,7 +23,7 @@ namespace geon {
 // N steps are N additions per coordinate instead of 28 metric evaluations each:
 // with the parameters of the reference's warp views a ray spends more than nine
 // tenths of its 20000 steps out there. A 96 x 54 view of 5000 steps: 487 ms
-// without, 34.5 ms with it.
+// without, 34.5 ms with it (25.0 since the other steps call alc_shape).
 template <int N>
 __device__ __forceinline__ bool alcubierre_flat_steps(const TraceLaunch& L, double y[8]) {
   const double dx = y[1] - L.M.p[3];
@@ -184,8 +184,8 @@ cudaError_t launch_trace_multi_fp64(const TraceLaunch* jobs, const MultiDesc& D,
 // (softfp.cuh), finiteness and magnitude tests on the high words, the quadrant
 // of theta from its high word. With one-warp blocks the Schwarzschild 256^2
 // view (r 30M, h 0.05, escape 100M) went from 247 to 151 ms, a 96 x 54
-// Alcubierre view of 5000 steps from 653 to 487 ms, bit for bit (and to 34.5 ms
-// with alcubierre_flat_steps).
+// Alcubierre view of 5000 steps from 653 to 487 ms, bit for bit (and to 25 ms
+// with alcubierre_flat_steps and alc_shape_called).
 template <int K, int SRC, int SINK>
 __global__ void __launch_bounds__(FP64_BLOCK, K == KIND_SCHWARZSCHILD ? 16 : 1) trace_fp64_kernel(const TraceLaunch L) {
   trace_loop<Fp64Stepper<K>, K, SRC, SINK>(L);
@@ -452,7 +452,8 @@ __global__ void pointwise_kernel(const MetricDesc M, int what, const double* __r
 // its warp is alone on its SM quarter. Here each lane evaluates one of them, the
 // values are exchanged by shuffles, and every lane forms the symbols (the same
 // expressions, so the same bits) and writes an eighth of them.
-// Whole host calls, one thread per point -> 8 lanes (us):
+// Whole host calls, one thread per point -> 8 lanes (us; at 8 points the left
+// figures are with a copy per buffer, 71 instead of 87 as one block: SmallCall):
 //                     8 points      608        9728       38912
 //   Alcubierre Gamma  87 -> 33    96 -> 47   130 -> 106  240 -> 274
 //   Alcubierre dg     74 -> 35    96 -> 48   133 -> 95   251 -> 240

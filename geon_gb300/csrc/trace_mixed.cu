@@ -844,13 +844,13 @@ struct MixedStepperAny : MixedCore<FEAT> {
 // step; 8 blocks of 128: <= 64 registers; 10: <= 51), trading registers (and
 // spills) for resident warps. Measured with the combined test and the
 // constant-bank constants, before and after: the 2^20-ray sweep 274 -> 269 ms
-// (cap 10), a 960 x 540 frame with 4 samples per pixel 29.4 -> 26.9 ms. What
-// bounds the step is not its instruction count any more (144 -> 139 of them,
-// and 126 in a version that tested only every fourth step ran no faster) but
-// the FP32 pipe with its register reads: 110 FP32 operations in ~158 cycles per
-// SM quarter; FFMA with three registers issues at 0.66 per cycle, and a mix of
-// FFMA, FADD and FMUL at 0.79. BLOCK is the block size (128 except for the
-// equatorial shadow kernel, whose autotuner also tries 64 and 256).
+// (cap 10), a 960 x 540 frame with 4 samples per pixel 29.4 -> 26.9 ms (25.9 with
+// the shading kernel of today). A sweep issues 0.88 instructions per cycle and SM
+// quarter, FMA pipe 70 % busy, the rest mostly dispatch stalls (three-register FFMA
+// issue at 0.66 per cycle, a mix of FFMA, FADD and FMUL at 0.79): ~143 instructions,
+// refills and starts of groups included, in ~162 cycles per step and quarter. BLOCK
+// is the block size (128 except for the equatorial shadow kernel, which also has 64
+// and 256, and 32 for trace_resident).
 template <int K, int SRC, int SINK, int MINB, int FEAT, int BLOCK = TRACE_BLOCK>
 __global__ void __launch_bounds__(BLOCK, MINB) trace_mixed_kernel(const TraceLaunch L) {
   constexpr int PL = (SRC == SRC_EQUATORIAL && K == KIND_SCHWARZSCHILD) ? FEAT_PLANAR : 0;
